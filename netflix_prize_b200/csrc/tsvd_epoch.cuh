@@ -81,8 +81,6 @@ __device__ __forceinline__ void gather_y8(const DeviceState& s, uint64_t n, Item
 
 // BF16 read copies of FP32 master rows (same padded layout, 2 bytes/element).
 struct Bf16Copies {
-    const __nv_bfloat16* ifeat;   // [I, Fs]
-    const __nv_bfloat16* qf0;     // [I, Fs] frequency-bin-0 rows of ifeat_freq
     const __nv_bfloat16* yfeat;   // [I, Fs]
     const __nv_bfloat16* pyc;     // [U, Fs] p_u + ycache_u
     const __nv_bfloat16* ufeat2;  // [U, Fs]

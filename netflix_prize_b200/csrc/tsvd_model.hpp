@@ -171,7 +171,7 @@ struct tsvd_model {
     tsvd::DevMem m_dyd_fix, m_qe0;
     tsvd::DevMem m_g_user, m_e_user, m_user_work, m_item_work, m_counters;
     // BF16 read copies (precision form)
-    tsvd::DevMem m_bf_ifeat, m_bf_qf0, m_bf_yfeat, m_bf_pyc, m_bf_ufeat2;
+    tsvd::DevMem m_bf_yfeat, m_bf_pyc, m_bf_ufeat2;
     tsvd::DevMem m_chunk_lo, m_item_chunk0, m_chunk_part, m_chunk_epart;
     tsvd::DevMem m_perm;          // [U] epoch order upload buffer
     // NSVD1 delta-sum passes: per chunk, the positions where the passes' user
@@ -184,7 +184,6 @@ struct tsvd_model {
     mutable tsvd::DevMem m_rows;
 
     std::vector<uint32_t> h_user_cnt;  // train counts (host copy)
-    uint32_t h_max_user_cnt = 0;       // the largest of them (made on first use)
     std::vector<uint32_t> h_split_bounds;  // user-block bounds of the delta-sum passes (m_chunk_split)
     std::vector<uint64_t> h_item_off;  // by-item offsets (host copy, made on first use)
     std::vector<uint64_t> h_ud_start;  // (user, day) offsets per user (host copy, made on first use)

@@ -567,8 +567,6 @@ void setup_params(tsvd_model* m) {
         zeros(m->m_counters, 64, st);
         m->m_perm.alloc(U * 4);
         if (m->opts.precision >= TSVD_PREC_BF16_READ) {
-            m->m_bf_ifeat.alloc((size_t)I * Fs * 2);
-            m->m_bf_qf0.alloc((size_t)I * Fs * 2);
             m->m_bf_yfeat.alloc((size_t)I * Fs * 2);
         }
         if (m->opts.precision >= TSVD_PREC_BF16_READ_ALL) {

@@ -22,7 +22,7 @@
 #include <vector>
 
 #include "rand_stream.hpp"
-#include "tsvd_epoch.cuh"
+#include "tsvd_chain.cuh"
 
 namespace tsvd {
 namespace {
@@ -43,34 +43,24 @@ __global__ void k_to_bf16(const float* __restrict__ src, uint64_t rows, uint32_t
 // The item rows a user-stratum rating reads: q_i and q^f_i of frequency bin fb.
 // qe0 = q_i + q^f_{i,0}: with low_memory the user stratum trains frequency bin
 // 0 only (src/tsvdx4p.rs:504-531) and reads the two rows only as this sum.
+// In the precision form both addends are rounded to BF16 first.
 __global__ void k_make_qe0(const float* __restrict__ ifeat, const float* __restrict__ ifeat_freq, uint64_t rows,
-                           uint32_t Fs, uint32_t NF, float* __restrict__ qe0) {
+                           uint32_t Fs, uint32_t NF, bool bf16, float* __restrict__ qe0) {
     const uint64_t n = rows * Fs;
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t r = e / Fs, c = e - r * Fs;
-        qe0[e] = ifeat[e] + ifeat_freq[r * NF * Fs + c];
+        const float q = ifeat[e], f = ifeat_freq[r * NF * Fs + c];
+        qe0[e] = bf16 ? __bfloat162float(__float2bfloat16_rn(q)) + __bfloat162float(__float2bfloat16_rn(f)) : q + f;
     }
 }
 
-void make_qe0(tsvd_model* m);
+void make_qe0(tsvd_model* m, bool bf16);
 
 
-template <int VPL, bool BF>
-__device__ __forceinline__ void item_rows(const DeviceState& s, const Bf16Copies& bf, uint32_t i, uint32_t fb, int lane,
-                                          float (&q)[VPL], float (&qf)[VPL]) {
-    if constexpr (BF) {
-        row_load_bf16<VPL>(bf.ifeat + (size_t)i * s.Fs, lane, q);
-        row_load_bf16<VPL>(bf.qf0 + (size_t)i * s.Fs, lane, qf);  // BF16 copies: low_memory, bin 0
-    } else {
-        Row<VPL>::load_nc(s.ifeat + (size_t)i * s.Fs, lane, q);
-        Row<VPL>::load_nc(s.ifeat_freq + ((size_t)i * s.NF + fb) * s.Fs, lane, qf);
-    }
-}
-
-// su gather with 8 rows in flight (FP32 or BF16 y rows), in the reference's order.
-template <int VPL, bool BF, class ItemOf>
-__device__ __forceinline__ void gather_y_ro(const DeviceState& s, const Bf16Copies& bf, uint64_t n, ItemOf item_of,
-                                            int lane, float (&su)[VPL], float& sub) {
+// su gather with 8 rows in flight, in the reference's order.
+template <int VPL, class ItemOf>
+__device__ __forceinline__ void gather_y_ro(const DeviceState& s, uint64_t n, ItemOf item_of, int lane,
+                                            float (&su)[VPL], float& sub) {
     constexpr int B = 8;
     for (uint64_t base = 0; base < n; base += 32) {
         const uint32_t cnt = (uint32_t)(n - base < 32 ? n - base : 32);
@@ -80,8 +70,7 @@ __device__ __forceinline__ void gather_y_ro(const DeviceState& s, const Bf16Copi
 #pragma unroll
             for (int q = 0; q < B; ++q) {
                 const uint32_t it = __shfl_sync(kFull, mine, j + q < cnt ? j + q : cnt - 1);
-                if constexpr (BF) row_load_bf16<VPL>(bf.yfeat + (size_t)it * s.Fs, lane, y[q]);
-                else Row<VPL>::load_nc(s.yfeat + (size_t)it * s.Fs, lane, y[q]);
+                Row<VPL>::load_nc(s.yfeat + (size_t)it * s.Fs, lane, y[q]);
                 yb[q] = __ldg(s.ybias + it);
             }
 #pragma unroll
@@ -94,13 +83,6 @@ __device__ __forceinline__ void gather_y_ro(const DeviceState& s, const Bf16Copi
             }
         }
     }
-}
-
-// The ordinal head's thresholds (lane-uniform); lr_t = 0 in every stratified
-// epoch, so they are constant within it.
-__device__ __forceinline__ void load_thresholds(const DeviceState& s, float (&th)[4]) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) th[k] = s.raw ? __ldg(s.thresholds + k) : 0.0f;
 }
 
 // err of a rating: score - residual, or with the ordinal head the gradient of
@@ -120,24 +102,18 @@ __device__ __forceinline__ void dyd_add(unsigned long long* row, int lane, const
 }
 
 // ---------------------------------------------------------------------------
-// User stratum (fit_epoch_user, src/tsvdx4p.rs:390-639). Item tables are
-// read-only here; the item rows of rating j+1 are requested before rating j
-// is used. With DAY (low_memory = false) each run of equal dates gets its
-// su_day from yfeat_day (the run's training items, then the day's pr items,
-// :500-527), the ratings add ufeat_day and su_day to p_u(t), ufeat_day is
-// trained (:604-611), and at the run's end its error sum over
-// sqrt(day count) goes to every item of the run as a yfeat_day delta
+// User stratum with the per-day terms (low_memory = false; fit_epoch_user,
+// src/tsvdx4p.rs:390-639; without them tsvd_user.cu). Item tables are read-only
+// here; the item rows of rating j+1 are requested before rating j is used. Each
+// run of equal dates gets its su_day from yfeat_day (the run's training items,
+// then the day's pr items, :500-527), the ratings add ufeat_day and su_day to
+// p_u(t), ufeat_day is trained (:604-611), and at the run's end its error sum
+// over sqrt(day count) goes to every item of the run as a yfeat_day delta
 // (:614-622).
 // ---------------------------------------------------------------------------
-// MINB blocks per SM. Three (a few registers spilled) pay off where the pass
-// is bound by its total work rather than by its longest user chains, which
-// every extra resident warp slows: 26.2 -> 24.2 ms at the full shape, f = 256,
-// but 10.0 -> 12.2 ms on 120,000 users with the same most active users.
-template <int VPL, bool BF, bool DAY, int MINB = 2>
-__global__ void __launch_bounds__(kThreads, MINB) k_user_strat(DeviceState s, EpochParams p, Bf16Copies bf,
-                                                         const uint32_t* __restrict__ order, uint32_t n_work) {
-    // FP32 with low_memory: the rating's item rows are read as their sum qe0
-    constexpr bool QE = !BF && !DAY;
+template <int VPL>
+__global__ void __launch_bounds__(kThreads, 2) k_user_strat(DeviceState s, EpochParams p,
+                                                            const uint32_t* __restrict__ order, uint32_t n_work) {
     const int lane = threadIdx.x & 31;
     const uint32_t Fs = s.Fs, T = s.T, NF = s.NF;
     float th[4];
@@ -165,11 +141,10 @@ __global__ void __launch_bounds__(kThreads, MINB) k_user_strat(DeviceState s, Ep
             for (int v = 0; v < VPL; ++v) su[v] = 0.0f;
             sub = 0.0f;
             const Rec* rr = s.rec + start;
-            gather_y_ro<VPL, BF>(s, bf, end - start, [&](uint64_t q) { return rec_id(__ldg(&rr[q].key)); }, lane, su,
-                                 sub);
+            gather_y_ro<VPL>(s, end - start, [&](uint64_t q) { return rec_id(__ldg(&rr[q].key)); }, lane, su, sub);
             if (p.full_su) {
                 const uint32_t* pp = s.pr_item + ps;
-                gather_y_ro<VPL, BF>(s, bf, pe - ps, [&](uint64_t q) { return __ldg(pp + q); }, lane, su, sub);
+                gather_y_ro<VPL>(s, pe - ps, [&](uint64_t q) { return __ldg(pp + q); }, lane, su, sub);
             }
 #pragma unroll
             for (int v = 0; v < VPL; ++v) su[v] = su[v] / norm;
@@ -188,8 +163,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_user_strat(DeviceState s, Ep
         float bb1 = lane + 32 < (int)T ? __ldcg(s.but_bin + (size_t)u * T + 32 + lane) : 0.0f;
         float sum_err = 0.0f;
         const float gb = s.gbias;
-        // the current run of equal dates (DAY)
-        float sud[DAY ? VPL : 1], seqd[DAY ? VPL : 1], pud[DAY ? VPL : 1];
+        // the current run of equal dates
+        float sud[VPL], seqd[VPL], pud[VPL];
         float norm_day = 1.0f;
         uint64_t run0 = 0, run1 = 0;
 
@@ -197,54 +172,50 @@ __global__ void __launch_bounds__(kThreads, MINB) k_user_strat(DeviceState s, Ep
             const uint32_t cnt = (uint32_t)(end - base < 32 ? end - base : 32);
             Rec mine{};
             if (lane < (int)cnt) mine = load_rec(s.rec + base + lane);
-            float qn[VPL], qfn[QE ? 1 : VPL];
+            float qn[VPL], qfn[VPL];
             auto fetch_item = [&](uint32_t key) {
-                if constexpr (QE) Row<VPL>::load_nc(s.qe0 + (size_t)rec_id(key) * Fs, lane, qn);
-                else item_rows<VPL, BF>(s, bf, rec_id(key), DAY ? rec_fbin(key) : 0u, lane, qn, qfn);
+                Row<VPL>::load_nc(s.ifeat + (size_t)rec_id(key) * Fs, lane, qn);
+                Row<VPL>::load_nc(s.ifeat_freq + ((size_t)rec_id(key) * NF + rec_fbin(key)) * Fs, lane, qfn);
             };
             fetch_item(__shfl_sync(kFull, mine.key, 0));
             for (uint32_t j = 0; j < cnt; ++j) {
                 const Rec r = shfl_rec(mine, j);
                 const uint32_t i = rec_id(r.key), tb = rec_tbin(r.key);
-                // low_memory: training uses frequency bin 0 (src/tsvdx4p.rs:504-531);
-                // with the per-day terms, the run's bin
-                const uint32_t fb = DAY ? rec_fbin(r.key) : 0u;
+                const uint32_t fb = rec_fbin(r.key);
                 const bool hud = r.ud < s.n_ud;
                 const uint64_t t = base + j;
-                if constexpr (DAY) {
-                    if (t == start || t > run1) {
-                        // a new run of equal dates (day_ranges, src/tx.rs:92-104)
-                        run0 = run1 = t;
-                        while (run1 + 1 < end && __ldg(&s.rec[run1 + 1].ud) == r.ud) ++run1;
+                if (t == start || t > run1) {
+                    // a new run of equal dates (day_ranges, src/tx.rs:92-104)
+                    run0 = run1 = t;
+                    while (run1 + 1 < end && __ldg(&s.rec[run1 + 1].ud) == r.ud) ++run1;
 #pragma unroll
-                        for (int v = 0; v < VPL; ++v) sud[v] = seqd[v] = 0.0f;
-                        float dummy = 0.0f;
-                        gather_rows8<VPL>(s.yfeat_day, nullptr, Fs, run1 - run0 + 1,
-                                          [&](uint64_t q) { return rec_id(__ldg(&s.rec[run0 + q].key)); }, lane, sud,
+                    for (int v = 0; v < VPL; ++v) sud[v] = seqd[v] = 0.0f;
+                    float dummy = 0.0f;
+                    gather_rows8<VPL>(s.yfeat_day, nullptr, Fs, run1 - run0 + 1,
+                                      [&](uint64_t q) { return rec_id(__ldg(&s.rec[run0 + q].key)); }, lane, sud,
+                                      dummy);
+                    float day_cnt = (float)(run1 - run0 + 1);
+                    if (p.full_su && hud) {
+                        const uint64_t off = s.ud_list_off[r.ud];
+                        const uint32_t pc = s.ud_pr_cnt[r.ud];
+                        gather_rows8<VPL>(s.yfeat_day, nullptr, Fs, pc,
+                                          [&](uint64_t q) { return __ldg(s.ud_list_item + off + q); }, lane, sud,
                                           dummy);
-                        float day_cnt = (float)(run1 - run0 + 1);
-                        if (p.full_su && hud) {
-                            const uint64_t off = s.ud_list_off[r.ud];
-                            const uint32_t pc = s.ud_pr_cnt[r.ud];
-                            gather_rows8<VPL>(s.yfeat_day, nullptr, Fs, pc,
-                                              [&](uint64_t q) { return __ldg(s.ud_list_item + off + q); }, lane, sud,
-                                              dummy);
-                            for (uint32_t c = 0; c < pc; ++c) day_cnt += 1.0f;
-                        }
-                        norm_day = sqrtf(day_cnt);
-#pragma unroll
-                        for (int v = 0; v < VPL; ++v) sud[v] = sud[v] / norm_day;
-                        if (p.has_ud && hud) Row<VPL>::load_cg(s.ufeat_day + (size_t)r.ud * Fs, lane, pud);
-                        else
-#pragma unroll
-                            for (int v = 0; v < VPL; ++v) pud[v] = 0.0f;
+                        for (uint32_t c = 0; c < pc; ++c) day_cnt += 1.0f;
                     }
+                    norm_day = sqrtf(day_cnt);
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) sud[v] = sud[v] / norm_day;
+                    if (p.has_ud && hud) Row<VPL>::load_cg(s.ufeat_day + (size_t)r.ud * Fs, lane, pud);
+                    else
+#pragma unroll
+                        for (int v = 0; v < VPL; ++v) pud[v] = 0.0f;
                 }
+            
                 float qe[VPL];  // q_i + q^f_{i,fb}
 #pragma unroll
                 for (int v = 0; v < VPL; ++v) {
-                    if constexpr (QE) qe[v] = qn[v];
-                    else qe[v] = qn[v] + qfn[v];
+                    qe[v] = qn[v] + qfn[v];
                 }
                 if (j + 1 < cnt) fetch_item(__shfl_sync(kFull, mine.key, j + 1));
                 const float ib = __ldg(s.ibias + i);
@@ -263,10 +234,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_user_strat(DeviceState s, Ep
 #pragma unroll
                 for (int v = 0; v < VPL; ++v) {
                     float pev = (pu[v] + su[v]) + dv * p2[v];
-                    if constexpr (DAY) {
-                        if (p.has_ud && hud) pev += pud[v];
-                        pev += sud[v];
-                    }
+                    if (p.has_ud && hud) pev += pud[v];
+                    pev += sud[v];
+                
                     part += qe[v] * pev;
                 }
                 const float dot = warp_sum(part);
@@ -289,23 +259,21 @@ __global__ void __launch_bounds__(kThreads, MINB) k_user_strat(DeviceState s, Ep
                     seq[v] += err * qe[v];
                     pu[v] = pk - p.lr_u * (err * qe[v] + p.reg_u * pk);
                     p2[v] = p2k - p.lr_u2 * (err * qe[v] * dv + p.reg_u2 * p2k);
-                    if constexpr (DAY) {
-                        seqd[v] += err * qe[v];
-                        if (p.has_ud && hud) pud[v] = pud[v] - p.lr_ud * (err * qe[v] + p.reg_ud * pud[v]);
-                    }
+                    seqd[v] += err * qe[v];
+                    if (p.has_ud && hud) pud[v] = pud[v] - p.lr_ud * (err * qe[v] + p.reg_ud * pud[v]);
+                
                 }
-                if constexpr (DAY) {
-                    if (t == run1) {
-                        // end of the run: ufeat_day back, and the run's yfeat_day
-                        // delta to each of its items (src/tsvdx4p.rs:614-622)
-                        if (p.has_ud && hud) Row<VPL>::store(s.ufeat_day + (size_t)r.ud * Fs, lane, pud);
-                        float gd[VPL];
+                if (t == run1) {
+                    // end of the run: ufeat_day back, and the run's yfeat_day
+                    // delta to each of its items (src/tsvdx4p.rs:614-622)
+                    if (p.has_ud && hud) Row<VPL>::store(s.ufeat_day + (size_t)r.ud * Fs, lane, pud);
+                    float gd[VPL];
 #pragma unroll
-                        for (int v = 0; v < VPL; ++v) gd[v] = seqd[v] / norm_day;
-                        for (uint64_t q2 = run0; q2 <= run1; ++q2)
-                            dyd_add<VPL>(s.dyd_fix + (size_t)rec_id(__ldg(&s.rec[q2].key)) * Fs, lane, gd);
-                    }
+                    for (int v = 0; v < VPL; ++v) gd[v] = seqd[v] / norm_day;
+                    for (uint64_t q2 = run0; q2 <= run1; ++q2)
+                        dyd_add<VPL>(s.dyd_fix + (size_t)rec_id(__ldg(&s.rec[q2].key)) * Fs, lane, gd);
                 }
+            
             }
         }
         Row<VPL>::store(s.ufeat + (size_t)u * Fs, lane, pu);
@@ -669,15 +637,6 @@ __device__ __forceinline__ void store_item_state(const DeviceState& s, uint32_t 
     if (lane + 32 < (int)T) s.bit_bin[(size_t)i * T + 32 + lane] = st.bt1;
     if (lane < (int)NF) s.ibias_freq[(size_t)i * NF + lane] = st.bf0;
     if (lane + 32 < (int)NF) s.ibias_freq[(size_t)i * NF + 32 + lane] = st.bf1;
-}
-
-// User-side scalars of one by-item rating: bu_t and cu_t (src/tsvdx4p.rs:690-708).
-__device__ __forceinline__ void user_scalars(const DeviceState& s, const Rec& r, float& bu_t, float& cu_t) {
-    const uint32_t u = rec_id(r.key), tb = rec_tbin(r.key);
-    const bool hud = r.ud < s.n_ud;
-    bu_t = __ldg(s.ubias + u) + __ldg(s.but_bin + (size_t)u * s.T + tb) + __ldg(s.alpha_u + u) * r.dev +
-           (hud ? __ldg(s.ubias_day + r.ud) : 0.0f) + __ldg(s.ycache_bias + u);
-    cu_t = __ldg(s.cu + u) + (hud ? __ldg(s.cut + r.ud) : 0.0f);
 }
 
 // The user-side rows of a by-item rating: p_u + ycache_u and p2_u.
@@ -1541,7 +1500,7 @@ __global__ void __launch_bounds__(kThreads) k_item_wide(DeviceState s, EpochPara
 
 void strat_launch_wide(tsvd_model* m, const EpochParams& p) {
     const DeviceState& s = m->d;
-    make_qe0(m);
+    make_qe0(m, false);
     {
         ProfScope ps(m, "user_pass_stratified");
         unsigned g = persistent_grid(k_user_strat_wide, 0);
@@ -1566,25 +1525,11 @@ void strat_launch_wide(tsvd_model* m, const EpochParams& p) {
     }
 }
 
-// Whether the user stratum of the whole user set is bound by its total work
-// rather than by its longest user chains: the ratings per warp at three blocks
-// per SM at least the most active user's count (1.66x at the full Netflix
-// shape, 0.41x on 120,000 users).
-bool user_stratum_work_bound(tsvd_model* m) {
-    if (m->h_max_user_cnt == 0)
-        for (uint32_t c : m->h_user_cnt) m->h_max_user_cnt = std::max(m->h_max_user_cnt, c);
-    int dev = 0, sms = 0;
-    TSVD_CUDA(cudaGetDevice(&dev));
-    TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const double warps = (double)sms * 3 * kWarps;
-    return (double)m->d.n_train / warps >= (double)std::max<uint32_t>(m->h_max_user_cnt, 1u);
-}
-
-void make_qe0(tsvd_model* m) {
+void make_qe0(tsvd_model* m, bool bf16) {
     const DeviceState& s = m->d;
     if (!s.qe0) return;
     const unsigned grid = (unsigned)std::min<uint64_t>(((uint64_t)s.n_items * s.Fs + 255) / 256, 148ull * 32);
-    k_make_qe0<<<grid, 256, 0, m->stream>>>(s.ifeat, s.ifeat_freq, s.n_items, s.Fs, s.NF, s.qe0);
+    k_make_qe0<<<grid, 256, 0, m->stream>>>(s.ifeat, s.ifeat_freq, s.n_items, s.Fs, s.NF, bf16, s.qe0);
     TSVD_CUDA(cudaGetLastError());
     m->launches++;
 }
@@ -1608,18 +1553,17 @@ void strat_launch(tsvd_model* m, const EpochParams& p, const Bf16Copies& bf) {
     DeviceState s = m->d;
     if (DAY || s.raw) s.heavy_min = 0xffffffffu;
     if (DAY) TSVD_CUDA(cudaMemsetAsync(s.dyd_fix, 0, (size_t)s.n_items * s.Fs * 8, m->stream));
-    if (!BF && !DAY) make_qe0(m);
+    if (!DAY) make_qe0(m, BF);
     {
         ProfScope ps(m, "user_pass_stratified");
-        if (!DAY && user_stratum_work_bound(m)) {
-            unsigned g = persistent_grid(k_user_strat<VPL, BF, DAY, 3>, 0);
-            k_user_strat<VPL, BF, DAY, 3><<<g, kThreads, 0, m->stream>>>(s, p, bf, s.user_work, s.n_users);
+        if constexpr (DAY) {
+            unsigned g = persistent_grid(k_user_strat<VPL>, 0);
+            k_user_strat<VPL><<<g, kThreads, 0, m->stream>>>(s, p, s.user_work, s.n_users);
+            TSVD_CUDA(cudaGetLastError());
+            m->launches++;
         } else {
-            unsigned g = persistent_grid(k_user_strat<VPL, BF, DAY>, 0);
-            k_user_strat<VPL, BF, DAY><<<g, kThreads, 0, m->stream>>>(s, p, bf, s.user_work, s.n_users);
+            launch_user_stratum(m, s, p, bf, s.user_work, s.n_users);
         }
-        TSVD_CUDA(cudaGetLastError());
-        m->launches++;
     }
     {
         ProfScope ps(m, "y_apply");
@@ -1676,16 +1620,15 @@ __global__ void k_reset_users(DeviceState s, const uint32_t* __restrict__ users,
 // which the next stratified epoch clears before its user stratum.)
 template <int VPL>
 void foldin_launch(tsvd_model* m, const EpochParams& p, const uint32_t* d_users, uint32_t n) {
-    make_qe0(m);
     if (m->d.dyd_fix) {
-        unsigned g = persistent_grid(k_user_strat<VPL, false, true>, 0);
-        k_user_strat<VPL, false, true><<<g, kThreads, 0, m->stream>>>(m->d, p, Bf16Copies{}, d_users, n);
+        unsigned g = persistent_grid(k_user_strat<VPL>, 0);
+        k_user_strat<VPL><<<g, kThreads, 0, m->stream>>>(m->d, p, d_users, n);
+        TSVD_CUDA(cudaGetLastError());
+        m->launches++;
     } else {
-        unsigned g = persistent_grid(k_user_strat<VPL, false, false>, 0);
-        k_user_strat<VPL, false, false><<<g, kThreads, 0, m->stream>>>(m->d, p, Bf16Copies{}, d_users, n);
+        make_qe0(m, false);
+        launch_user_stratum(m, m->d, p, Bf16Copies{}, d_users, n);
     }
-    TSVD_CUDA(cudaGetLastError());
-    m->launches++;
 }
 
 // ---------------------------------------------------------------------------
@@ -1698,18 +1641,24 @@ template <int VPL, bool DAY>
 void shard_user_launch(tsvd_model* m, const EpochParams& p, const uint32_t* work, uint32_t n, uint32_t u_lo,
                        uint32_t u_hi, float* sums, float* sums_e) {
     const DeviceState& s = m->d;
-    if (!DAY) make_qe0(m);
+    if (!DAY) make_qe0(m, false);
     {
         ProfScope ps(m, "user_pass_stratified");
         if (s.Fs > kSlice) {
             unsigned g = persistent_grid(k_user_strat_wide, 0);
             k_user_strat_wide<<<g, kThreads, 0, m->stream>>>(s, p, work, n);
+            TSVD_CUDA(cudaGetLastError());
+            m->launches++;
         } else {
-            unsigned g = persistent_grid(k_user_strat<VPL, false, DAY>, 0);
-            k_user_strat<VPL, false, DAY><<<g, kThreads, 0, m->stream>>>(s, p, Bf16Copies{}, work, n);
+            if constexpr (DAY) {
+                unsigned g = persistent_grid(k_user_strat<VPL>, 0);
+                k_user_strat<VPL><<<g, kThreads, 0, m->stream>>>(s, p, work, n);
+                TSVD_CUDA(cudaGetLastError());
+                m->launches++;
+            } else {
+                launch_user_stratum(m, s, p, Bf16Copies{}, work, n);
+            }
         }
-        TSVD_CUDA(cudaGetLastError());
-        m->launches++;
     }
     ProfScope ps(m, "y_apply");
     y_partial_passes<VPL>(m, s, u_lo, u_hi);
@@ -1770,11 +1719,7 @@ void stratified_epoch(tsvd_model* m, const EpochParams& p) {
     Bf16Copies bf{};
     if (prec >= TSVD_PREC_BF16_READ) {
         ProfScope ps(m, "bf16_copies");
-        to_bf16(m, s.ifeat, s.n_items, s.Fs, m->m_bf_ifeat.p);
-        to_bf16(m, s.ifeat_freq, s.n_items, (uint64_t)s.NF * s.Fs, m->m_bf_qf0.p);
         to_bf16(m, s.yfeat, s.n_items, s.Fs, m->m_bf_yfeat.p);
-        bf.ifeat = m->m_bf_ifeat.as<__nv_bfloat16>();
-        bf.qf0 = m->m_bf_qf0.as<__nv_bfloat16>();
         bf.yfeat = m->m_bf_yfeat.as<__nv_bfloat16>();
     }
     if (prec >= TSVD_PREC_BF16_READ_ALL) {

@@ -1,0 +1,111 @@
+"""The strata's blocked chains at the sizes where they can go wrong, against the
+oracle's tsvdx4p epoch (the reference's src/tsvdx4p.rs:390-762).
+
+Tolerance: a parameter is a sum of at most a few hundred updates of at most
+|lr x| ~ 1e-2 each, in FP32 in both, in another order; 2e-5 absolute is the
+bound every other parity test of one epoch holds.
+"""
+import numpy as np
+import pytest
+
+from netflix_prize_b200.abi import PREC_FP32
+from netflix_prize_b200.config import OrdinalHeadConfig, run_lm
+from netflix_prize_b200.data import Dataset, MaskedDataset
+from netflix_prize_b200.encoder import foldin
+from netflix_prize_b200.model import TxModel
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+PARAMS = ["ubias", "ibias", "ufeat", "ufeat2", "ifeat", "yfeat", "alpha_u", "but_bin", "bit_bin", "ybias",
+          "ubias_day", "ibias_freq", "ifeat_freq", "cu", "cut"]
+
+
+def counted_sets(counts, n_items, seed):
+    """Users with exactly these numbers of training ratings, several on a day,
+    and two query pairs each."""
+    rng = np.random.default_rng(seed)
+    u, i, d, pu, pi, pd = [], [], [], [], [], []
+    for k, n in enumerate(counts):
+        items = np.sort(rng.choice(n_items, size=n + 2, replace=False))
+        days = rng.integers(0, 1500, size=max(1, n // 3))
+        q = rng.permutation(n + 2)
+        u += [k] * n
+        i += list(items[np.sort(q[:n])])
+        d += list(rng.choice(days, size=n))
+        pu += [k] * 2
+        pi += list(items[q[n:]])
+        pd += list(rng.choice(days, size=2))
+    tr = Dataset.from_ratings(u, i, rng.integers(1, 6, len(u)), d, len(counts), n_items, "counted_tr")
+    o = np.lexsort((np.array(pu), np.array(pi)))
+    pr = Dataset.from_ratings(np.array(pu)[o], np.array(pi)[o], rng.integers(1, 6, len(pu)), np.array(pd)[o],
+                              len(counts), n_items, "counted_pr")
+    return tr, pr
+
+
+def check_epochs(tr, pr, cfg, epochs=2, **kw):
+    o = po.OracleModel(tr, MaskedDataset(pr), cfg)
+    g = TxModel(tr, MaskedDataset(pr), cfg, precision=PREC_FP32, **kw)
+    for e in range(1, epochs + 1):
+        o.fit_epoch(e, po.SCHED_P, nsvd_norm_exp=1.0, n_threads=1)
+        g.fit_epoch(tr, pr, e)
+    names = PARAMS if cfg.low_memory else PARAMS + ["yfeat_day", "ufeat_day"]
+    for n in names:
+        a = np.asarray(g.get_param(n), np.float64).ravel()
+        b = np.asarray(o.get_param(n), np.float64).ravel()
+        if a.size:
+            assert np.max(np.abs(a - b) - 1e-5 * np.abs(b)) < 2e-5, n
+
+
+@pytest.mark.parametrize("f", [0, 20, 33, 64, 96, 130, 190, 224, 256])
+def test_user_stratum_at_the_edges_of_its_pairs_and_chunks(f):
+    """Users with 1, 2, 3 ratings (a pair, a pair and a half), with a chunk of
+    32 less and more one, and with a count past the ring of rows; the time-bin
+    biases trained; every row layout."""
+    counts = [1, 2, 3, 5, 6, 7, 8, 9, 31, 32, 33, 63, 64, 65, 97, 150]
+    tr, pr = counted_sets(counts, 200, 3 + f)
+    check_epochs(tr, pr, run_lm(f, 2, n_time_bins=48).replace(lr_tu=0.001, reset_u_epoch=2 if f == 64 else 1024))
+
+
+def user_pass_ordinal(g, tr, cfg, u):
+    """One user's ordinal-head pass over its training ratings, items frozen, in
+    float64 (src/tsvdx4p.rs:535-613 with the head's gradient, src/lib.rs:562-598)."""
+    P = {n: np.asarray(g.get_param(n), np.float64) for n in PARAMS + ["ycache", "ycache_bias", "tu_mean"]}
+    th = np.array(cfg.ordinal_head.th_init)
+    pu, p2, ub, al, cu = P["ufeat"][u], P["ufeat2"][u], P["ubias"][u], P["alpha_u"][u], P["cu"][u]
+    but, bud = P["but_bin"][u].copy(), {}
+    for t in np.nonzero(tr.user_idxs == u)[0]:
+        i, day = tr.item_idxs[t], int(tr.dates[t])
+        tb = min(day * cfg.n_time_bins // (int(tr.dates.max()) + 1), cfg.n_time_bins - 1)
+        dt = day - P["tu_mean"][u]
+        dv = np.sign(dt) * abs(dt) ** np.float64(np.float32(cfg.beta))
+        qe = P["ifeat"][i] + P["ifeat_freq"][i * cfg.n_freq_bins]
+        bi = P["ibias"][i] + P["bit_bin"][i, tb] + P["ibias_freq"][i, 0]
+        x = (float(g.get_param("gbias")) + ub + but[tb] + al * dv + bud.get(day, 0.0) + P["ycache_bias"][u] + bi * cu
+             + qe @ (pu + P["ycache"][u] + dv * p2))
+        f = np.concatenate([[0.0], 1 / (1 + np.exp(-(th - x))), [1.0]])
+        y = int(tr.raw_ratings[t])
+        e = (f[y] * (1 - f[y]) - f[y - 1] * (1 - f[y - 1])) / max(f[y] - f[y - 1], 1e-6)
+        ub, al = ub - cfg.lr_ub * e, al - cfg.lr_ta * e * dv
+        but[tb] -= cfg.lr_tu * e
+        bud[day] = bud.get(day, 0.0) - cfg.lr_ubd * e
+        cu = cu - cfg.lr_cu * (e * bi + cfg.reg_cu * (cu - 1))
+        pu, p2 = (pu - cfg.lr_u * (e * qe + cfg.reg_u * pu), p2 - cfg.lr_u2 * (e * qe * dv + cfg.reg_u2 * p2))
+    return pu, p2, ub, al, cu, but
+
+
+@pytest.mark.parametrize("f", [20, 64, 160])
+def test_user_stratum_with_the_ordinal_head(f):
+    """The head's gradient is not linear in the score: a pair's second rating
+    must see the first one's update. A fold-in pass is the user stratum alone."""
+    counts = [1, 2, 3, 31, 33, 64, 90]
+    tr, pr = counted_sets(counts, 120, 9)
+    cfg = run_lm(f, 1, n_time_bins=30).replace(
+        lr_tu=0.001, sigma_u=0.1, sigma_i=0.1, ordinal_head=OrdinalHeadConfig((0.5, 1.25, 3.75, 5.5), 0.001, 0.0, 0.0))
+    g = TxModel(tr, MaskedDataset(pr), cfg)
+    g.rebuild_ycache()
+    want = [user_pass_ordinal(g, tr, cfg, u) for u in range(len(counts))]
+    foldin(g, np.arange(len(counts)), 1)
+    for n, k in (("ufeat", 0), ("ufeat2", 1), ("ubias", 2), ("alpha_u", 3), ("cu", 4), ("but_bin", 5)):
+        a = np.asarray(g.get_param(n), np.float64)
+        assert np.max(np.abs(a - np.array([w[k] for w in want]))) < 2e-5, n
