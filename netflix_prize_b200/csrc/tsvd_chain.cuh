@@ -160,6 +160,61 @@ struct Vec {
     }
 };
 
+// su += y_j (and sub += b_j, when yb is given) for the items item_of(0 .. n-1),
+// added in order: rows of the table y, or of its BF16 copy. kRows rows are asked
+// for together; the loop over whole groups has no bounds checks, so a row costs
+// its loads, its adds and four instructions more.
+template <int VPL, bool BF, class ItemOf>
+__device__ __forceinline__ void sum_rows(const float* __restrict__ y, const __nv_bfloat16* __restrict__ ybf,
+                                         const float* __restrict__ yb, uint32_t Fs, uint64_t n, ItemOf item_of, int lane,
+                                         Vec<VPL>& su, float& sub) {
+    constexpr int kRows = VPL >= 5 ? 8 : VPL >= 2 ? 16 : 32;
+    auto row = [&](uint32_t it, Vec<VPL>& x) {
+        if constexpr (BF) x.load_bf16(ybf + (size_t)it * Fs, lane);
+        else x.load_nc(y + (size_t)it * Fs, lane);
+    };
+    // a chunk's 32 items, one per lane, a chunk ahead
+    uint32_t next = (uint64_t)lane < n ? item_of(lane) : 0u;
+    for (uint64_t base = 0; base < n; base += 32) {
+        const uint32_t cnt = (uint32_t)(n - base < 32 ? n - base : 32);
+        const uint32_t mine = next;
+        const float b = yb ? __ldg(yb + mine) : 0.0f;
+        if (base + 32 + lane < n) next = item_of(base + 32 + lane);
+        uint32_t j = 0;
+#pragma unroll 1
+        for (; j + kRows <= cnt; j += kRows) {
+            Vec<VPL> x[kRows];
+#pragma unroll
+            for (int q = 0; q < kRows; ++q) row(__shfl_sync(kFull, mine, j + q), x[q]);
+#pragma unroll
+            for (int q = 0; q < kRows; ++q) {
+                su.add(x[q]);
+                sub += __shfl_sync(kFull, b, j + q);
+            }
+        }
+        if (kRows > 4) {
+#pragma unroll 1
+            for (; j + 4 <= cnt; j += 4) {
+                Vec<VPL> x[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) row(__shfl_sync(kFull, mine, j + q), x[q]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    su.add(x[q]);
+                    sub += __shfl_sync(kFull, b, j + q);
+                }
+            }
+        }
+#pragma unroll 1
+        for (; j < cnt; ++j) {
+            Vec<VPL> x;
+            row(__shfl_sync(kFull, mine, j), x);
+            su.add(x);
+            sub += __shfl_sync(kFull, b, j);
+        }
+    }
+}
+
 // The ordinal head's thresholds (lane-uniform); lr_t = 0 in every stratified
 // epoch, so they are constant within it.
 __device__ __forceinline__ void load_thresholds(const DeviceState& s, float (&th)[4]) {

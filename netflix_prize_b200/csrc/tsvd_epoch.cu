@@ -17,7 +17,7 @@
 #include <cstring>
 
 #include "rand_stream.hpp"
-#include "tsvd_epoch.cuh"
+#include "tsvd_chain.cuh"
 
 namespace tsvd {
 
@@ -359,70 +359,45 @@ __global__ void __launch_bounds__(kThreads, 2) k_hog_batched(const DeviceState* 
 
 // ---------------------------------------------------------------------------
 // ycache[u] = |N(u)|^-1/2 sum over train and pr items (rebuild_ycache,
-// src/tx.rs:391-418): train items in rating order, then pr items in pr order.
+// src/tx.rs:391-418): train items in rating order, then pr items in pr order. One
+// warp per user. At the full shape, f = 256, bound by what L2 delivers to the SMs
+// (a row is 1 KB; 17 TB/s of rows), elsewhere by the most active users' sums,
+// which is why several rows are asked for at a time, users come most active
+// first, and the registers are left to three blocks per SM: 100,480,507 ratings,
+// f = 256, 12.0 -> 5.9 ms; 25 M ratings, f = 64, 3.5 -> 1.1 ms (one B200, CUDA
+// events; with four blocks per SM the row groups spill: 7.1 and 3.0 ms).
 // ---------------------------------------------------------------------------
-template <int VPL>
-__global__ void __launch_bounds__(kThreads) k_rebuild_ycache(DeviceState s, const __nv_bfloat16* __restrict__ ybf,
-                                                              float* __restrict__ pyc);
-
-template <int VPL>
+template <int VPL, bool BF>
 __device__ __forceinline__ void rebuild_user(const DeviceState& s, const __nv_bfloat16* __restrict__ ybf, uint32_t u,
                                              int lane, float* __restrict__ pyc) {
-    constexpr int B = 8;  // rows in flight
     const uint64_t a = s.user_off[u], b = s.user_off[u + 1];
     const uint64_t pa = s.pr_off[u], pb = s.pr_off[u + 1];
     const uint64_t ntr = b - a, n = ntr + (pb - pa);
     const int32_t cnt_all = s.user_cnt_tr[u] + s.user_cnt_pr[u];
+    // the item of entry q of N(u): training ratings first, then pr items
+    auto item_at = [&](uint64_t q) -> uint32_t {
+        return q < ntr ? rec_id(__ldg(&s.rec[a + q].key)) : __ldg(s.pr_item + pa + (q - ntr));
+    };
     // rows wider than 32 * VPL columns (n_feat > 256) in slices of 32 * VPL
     for (uint32_t c0 = 0; c0 < s.Fs; c0 += 32 * VPL) {
-        float su[VPL];
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) su[v] = 0.0f;
+        Vec<VPL> su;
+        su.zero();
         float sub = 0.0f;
-        // the item of entry q of N(u): training ratings first, then pr items
-        auto item_at = [&](uint64_t q) -> uint32_t {
-            return q < ntr ? rec_id(__ldg(&s.rec[a + q].key)) : __ldg(s.pr_item + pa + (q - ntr));
-        };
-        // each chunk's 32 items are loaded one chunk ahead (one per lane)
-        uint32_t nxt = (uint64_t)lane < n ? item_at(lane) : 0u;
-        for (uint64_t base = 0; base < n; base += 32) {
-            const uint32_t cnt = (uint32_t)(n - base < 32 ? n - base : 32);
-            const uint32_t mine = nxt;
-            if (base + 32 + lane < n) nxt = item_at(base + 32 + lane);
-            for (uint32_t j = 0; j < cnt; j += B) {
-                float y[B][VPL], yb[B];
-#pragma unroll
-                for (int t = 0; t < B; ++t) {
-                    const uint32_t it = __shfl_sync(kFull, mine, j + t < cnt ? j + t : cnt - 1);
-                    if (ybf) row_load_bf16<VPL>(ybf + (size_t)it * s.Fs + c0, lane, y[t]);
-                    else Row<VPL>::load_nc(s.yfeat + (size_t)it * s.Fs + c0, lane, y[t]);
-                    yb[t] = c0 == 0 ? __ldg(s.ybias + it) : 0.0f;
-                }
-#pragma unroll
-                for (int t = 0; t < B; ++t) {
-                    if (j + t < cnt) {
-#pragma unroll
-                        for (int v = 0; v < VPL; ++v) su[v] += y[t][v];
-                        sub += yb[t];
-                    }
-                }
-            }
-        }
+        sum_rows<VPL, BF>(s.yfeat + c0, BF ? ybf + c0 : nullptr, c0 == 0 ? s.ybias : nullptr, s.Fs, n, item_at, lane, su,
+                          sub);
         if (cnt_all > 0) {
             const float nrm = sqrtf((float)cnt_all);
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) su[v] = su[v] / nrm;
+            su.divide(nrm);
             sub = sub / nrm;
         }
-        Row<VPL>::store(s.ycache + (size_t)u * s.Fs + c0, lane, su);
+        su.store_cg(s.ycache + (size_t)u * s.Fs + c0, lane);
         if (lane == 0 && c0 == 0) s.ycache_bias[u] = sub;
         if (pyc) {
             // p_u + ycache_u, the user-side sum every item-stratum rating of u reads
-            float pu[VPL];
-            Row<VPL>::load_cg(s.ufeat + (size_t)u * s.Fs + c0, lane, pu);
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) pu[v] = pu[v] + su[v];
-            Row<VPL>::store(pyc + (size_t)u * s.Fs + c0, lane, pu);
+            Vec<VPL> pu;
+            pu.load_cg(s.ufeat + (size_t)u * s.Fs + c0, lane);
+            pu.add(su);
+            pu.store_cg(pyc + (size_t)u * s.Fs + c0, lane);
         }
     }
 }
@@ -437,25 +412,27 @@ __global__ void __launch_bounds__(kThreads) k_rebuild_batched(const DeviceState*
         const uint32_t mk = (uint32_t)(w / n_users), u = (uint32_t)(w - (uint64_t)mk * n_users);
         const DeviceState& s = states[mk];
         switch (s.Fs >> 5) {
-            case 1: rebuild_user<1>(s, nullptr, u, lane, nullptr); break;
-            case 2: rebuild_user<2>(s, nullptr, u, lane, nullptr); break;
-            case 3: rebuild_user<3>(s, nullptr, u, lane, nullptr); break;
-            case 4: rebuild_user<4>(s, nullptr, u, lane, nullptr); break;
-            case 5: rebuild_user<5>(s, nullptr, u, lane, nullptr); break;
-            case 6: rebuild_user<6>(s, nullptr, u, lane, nullptr); break;
-            case 7: rebuild_user<7>(s, nullptr, u, lane, nullptr); break;
-            default: rebuild_user<8>(s, nullptr, u, lane, nullptr); break;
+            case 1: rebuild_user<1, false>(s, nullptr, u, lane, nullptr); break;
+            case 2: rebuild_user<2, false>(s, nullptr, u, lane, nullptr); break;
+            case 3: rebuild_user<3, false>(s, nullptr, u, lane, nullptr); break;
+            case 4: rebuild_user<4, false>(s, nullptr, u, lane, nullptr); break;
+            case 5: rebuild_user<5, false>(s, nullptr, u, lane, nullptr); break;
+            case 6: rebuild_user<6, false>(s, nullptr, u, lane, nullptr); break;
+            case 7: rebuild_user<7, false>(s, nullptr, u, lane, nullptr); break;
+            default: rebuild_user<8, false>(s, nullptr, u, lane, nullptr); break;
         }
     }
 }
 
-template <int VPL>
-__global__ void __launch_bounds__(kThreads) k_rebuild_ycache(DeviceState s, const __nv_bfloat16* __restrict__ ybf,
+// Users in processing order, the most active first: their sums are the longest.
+template <int VPL, bool BF>
+__global__ void __launch_bounds__(kThreads, 3) k_rebuild_ycache(DeviceState s, const __nv_bfloat16* __restrict__ ybf,
                                                               float* __restrict__ pyc) {
     const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * kWarps;
-    for (uint32_t u = blockIdx.x * kWarps + (threadIdx.x >> 5); u < s.n_users; u += warps)
-        rebuild_user<VPL>(s, ybf, u, lane, pyc);
+    // neighbouring ranks on different SMs
+    for (uint32_t k = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; k < s.n_users; k += warps)
+        rebuild_user<VPL, BF>(s, ybf, s.user_work[k], lane, pyc);
 }
 
 // ---------------------------------------------------------------------------
@@ -473,8 +450,13 @@ void launch_hog_pass(tsvd_model* m, const EpochParams& p, const uint32_t* order)
 
 template <int VPL>
 void launch_rebuild(tsvd_model* m, const __nv_bfloat16* ybf, float* pyc) {
-    unsigned g = persistent_grid(k_rebuild_ycache<VPL>, 0);
-    k_rebuild_ycache<VPL><<<g, kThreads, 0, m->stream>>>(m->d, ybf, pyc);
+    if (ybf) {
+        unsigned g = persistent_grid(k_rebuild_ycache<VPL, true>, 0);
+        k_rebuild_ycache<VPL, true><<<g, kThreads, 0, m->stream>>>(m->d, ybf, pyc);
+    } else {
+        unsigned g = persistent_grid(k_rebuild_ycache<VPL, false>, 0);
+        k_rebuild_ycache<VPL, false><<<g, kThreads, 0, m->stream>>>(m->d, ybf, pyc);
+    }
     TSVD_CUDA(cudaGetLastError());
     m->launches++;
 }

@@ -35,35 +35,6 @@ constexpr int kUThreads = 128;
 constexpr int kRingRows = 8;    // slots of a warp's ring
 constexpr int kAheadRows = 6;   // ratings asked for ahead (even, < kRingRows - 1)
 
-// su = the y rows of the user's n items in order (FP32 or BF16 y rows).
-template <int VPL, class ItemOf>
-__device__ __forceinline__ void gather_y(const DeviceState& s, const Bf16Copies& bf, uint64_t n, ItemOf item_of, int lane,
-                                         Vec<VPL>& su, float& sub) {
-    constexpr int B = 4;
-    for (uint64_t base = 0; base < n; base += 32) {
-        const uint32_t cnt = (uint32_t)(n - base < 32 ? n - base : 32);
-        const uint32_t mine = lane < (int)cnt ? item_of(base + lane) : 0u;
-        for (uint32_t j = 0; j < cnt; j += B) {
-            Vec<VPL> y[B];
-            float yb[B];
-#pragma unroll
-            for (int q = 0; q < B; ++q) {
-                const uint32_t it = __shfl_sync(kFull, mine, j + q < cnt ? j + q : cnt - 1);
-                if (bf.yfeat) y[q].load_bf16(bf.yfeat + (size_t)it * s.Fs, lane);
-                else y[q].load_nc(s.yfeat + (size_t)it * s.Fs, lane);
-                yb[q] = __ldg(s.ybias + it);
-            }
-#pragma unroll
-            for (int q = 0; q < B; ++q) {
-                if (j + q < cnt) {
-                    su.add(y[q]);
-                    sub += yb[q];
-                }
-            }
-        }
-    }
-}
-
 // CTAs per SM the registers are bounded for: the most that spill nothing (at f =
 // 256 one more CTA, with 56 bytes spilled, measured 17.5 against 16.0 ms).
 constexpr int user_ctas(int vpl) { return vpl >= 7 ? 4 : vpl >= 5 ? 5 : vpl >= 3 ? 6 : 7; }
@@ -108,10 +79,16 @@ __global__ void __launch_bounds__(kUThreads, user_ctas(VPL)) k_user_pairs(Device
             su.zero();
             sub = 0.0f;
             const Rec* rr = s.rec + start;
-            gather_y<VPL>(s, bf, end - start, [&](uint64_t q) { return rec_id(__ldg(&rr[q].key)); }, lane, su, sub);
-            if (p.full_su) {
-                const uint32_t* pp = s.pr_item + ps;
-                gather_y<VPL>(s, bf, pe - ps, [&](uint64_t q) { return __ldg(pp + q); }, lane, su, sub);
+            const uint32_t* pp = s.pr_item + ps;
+            auto train = [&](uint64_t q) { return rec_id(__ldg(&rr[q].key)); };
+            auto probe = [&](uint64_t q) { return __ldg(pp + q); };
+            const uint64_t n_pr = p.full_su ? pe - ps : 0;
+            if (bf.yfeat) {
+                sum_rows<VPL, true>(nullptr, bf.yfeat, s.ybias, Fs, end - start, train, lane, su, sub);
+                sum_rows<VPL, true>(nullptr, bf.yfeat, s.ybias, Fs, n_pr, probe, lane, su, sub);
+            } else {
+                sum_rows<VPL, false>(s.yfeat, nullptr, s.ybias, Fs, end - start, train, lane, su, sub);
+                sum_rows<VPL, false>(s.yfeat, nullptr, s.ybias, Fs, n_pr, probe, lane, su, sub);
             }
             su.divide(norm);
             sub = sub / norm;

@@ -109,3 +109,20 @@ def test_user_stratum_with_the_ordinal_head(f):
     for n, k in (("ufeat", 0), ("ufeat2", 1), ("ubias", 2), ("alpha_u", 3), ("cu", 4), ("but_bin", 5)):
         a = np.asarray(g.get_param(n), np.float64)
         assert np.max(np.abs(a - np.array([w[k] for w in want]))) < 2e-5, n
+
+
+@pytest.mark.parametrize("f", [20, 64, 100, 160, 200, 256, 300])
+def test_ycache_rebuild_is_bitwise_at_the_edges_of_its_row_groups(f):
+    """The sums run over groups of 32, 16 or 8 rows, then four, then one, and a
+    chunk of 32 items ahead; every add is in the reference's order."""
+    counts = [1, 2, 3, 4, 5, 6, 7, 9, 13, 14, 15, 28, 29, 30, 31, 32, 45, 61, 62, 63, 94, 95]
+    tr, pr = counted_sets(counts, 150, 17)
+    cfg = run_lm(f, 1, n_time_bins=30)
+    o, g = po.OracleModel(tr, MaskedDataset(pr), cfg), TxModel(tr, MaskedDataset(pr), cfg)
+    yb = np.random.default_rng(5).normal(0, 0.1, tr.n_items).astype(np.float32)
+    for m in (o, g):
+        m.set_param("ybias", yb)
+        m.rebuild_ycache()
+    for n in ("ycache", "ycache_bias"):
+        a = np.asarray(g.get_param(n), np.float32).ravel()
+        assert np.array_equal(a.view(np.uint32), np.asarray(o.get_param(n), np.float32).ravel().view(np.uint32)), n
