@@ -236,4 +236,8 @@ __device__ __forceinline__ void user_scalars(const DeviceState& s, const Rec& r,
 void launch_user_stratum(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf,
                          const uint32_t* work, uint32_t n);
 
+// The item stratum of rows up to 256 columns (tsvd_item.cu): the items of
+// s.item_work, heaviest first.
+void launch_item_stratum(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf);
+
 }  // namespace tsvd

@@ -91,6 +91,8 @@ tsvd_model* make_variant(const tsvd_model* base, const tsvd_config& cfg) {
     m->d.F = (uint32_t)cfg.n_feat;
     m->d.Fs = (uint32_t)((cfg.n_feat + 31) / 32 * 32);
     m->h_user_cnt = base->h_user_cnt;
+    m->d.heavy_min = tsvd::heavy_min_for(m);
+    m->d.rounded_decay_min = tsvd::rounded_decay_min_for(m);
     tsvd::setup_params(m);
     return m;
 }

@@ -132,6 +132,7 @@ struct DeviceState {
     uint32_t* counters;         // [8] dynamic work counters
     // fixed-size chunks of the by-item index (deterministic split reductions)
     uint32_t heavy_min;  // item stratum: items with at least this many ratings take a whole block
+    uint32_t rounded_decay_min;  // item stratum: items whose rows decay by factors rounded to FP32
     uint32_t n_chunks;
     const uint64_t* chunk_lo;      // [n_chunks + 1] start of each chunk in irec; last = n_train
     const uint32_t* item_chunk0;   // [I+1] first chunk of each item
@@ -200,6 +201,9 @@ namespace tsvd {
 // setup (tsvd_setup.cu)
 void setup_model(tsvd_model* m, const tsvd_dataset_view& tr, const tsvd_dataset_view& pr);
 void setup_params(tsvd_model* m);
+// item stratum: ratings from which an item is heavy, and from which its rows decay by FP32 factors
+uint32_t heavy_min_for(const tsvd_model* m);
+uint32_t rounded_decay_min_for(const tsvd_model* m);
 // seeded normal init on the device (tsvd_init.cu)
 struct NormalTable {
     float* dst;       // rows x stride floats; columns cols..stride-1 are zeroed

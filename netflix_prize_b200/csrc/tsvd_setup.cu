@@ -178,6 +178,29 @@ std::vector<uint32_t> heaviest_first(const C* cnt, uint32_t n) {
     return out;
 }
 
+// Heavy items take a CTA each, the others a warp each: a rating then costs the
+// GPU less, but its chain is longer. The line is where a light item's chain is
+// about as long as the pass, in shares of the ratings an SM gets: rows up to 128
+// columns (25 M ratings, f = 64) 9.9 ms at a quarter (42,000), 11.5 at 20,000,
+// 13.0 at 60,000; wider rows (f = 256) 16.9 ms at a twentieth (8,000), 19.9 at
+// 20,000, and 60.4 at 32,768 of 100 M.
+uint32_t heavy_min_for(const tsvd_model* m) {
+    if (m->opts.heavy_item_ratings > 0) return (uint32_t)m->opts.heavy_item_ratings;
+    int sms = 0;
+    TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
+    const uint64_t share = m->d.n_train / ((m->d.Fs > 128 ? 20 : 4) * (uint64_t)sms);
+    return (uint32_t)std::min<uint64_t>(0x7fffffffu, std::max<uint64_t>(64, share));
+}
+
+// A row's decay by x - lr reg x is added as (a - 1) x, a = 1 - lr reg, which keeps
+// lr reg's own digits. Items of at least this many ratings multiply by a rounded to
+// FP32 instead (for q^f rows, lr reg = 3.5e-8 becomes 6.0e-8): a model trained on
+// from a saved state, or compared with one, keeps the rows it has had.
+uint32_t rounded_decay_min_for(const tsvd_model* m) {
+    if (!m->cfg.low_memory || m->cfg.has_ordinal_head) return 0xffffffffu;
+    return m->opts.heavy_item_ratings > 0 ? (uint32_t)m->opts.heavy_item_ratings : 32768u;
+}
+
 void setup_model(tsvd_model* m, const tsvd_dataset_view& tr, const tsvd_dataset_view& pr) {
     const tsvd_config& c = m->cfg;
     cudaStream_t st = m->stream;
@@ -315,11 +338,10 @@ void setup_model(tsvd_model* m, const tsvd_dataset_view& tr, const tsvd_dataset_
     const uint32_t Fs = F == 0 ? 32u : F <= 256 ? (F + 31) / 32 * 32 : (F + 255) / 256 * 256;
     s.n_users = U; s.n_items = I; s.F = F; s.Fs = Fs;
     s.T = (uint32_t)c.n_time_bins; s.NF = (uint32_t)c.n_freq_bins;
-    // Heavy items run as rounds on a whole block; below the threshold a warp
-    // per item is cheaper per rating, as long as its chain stays shorter than
-    // the hottest item's (32768 measured best at the full Netflix shape).
-    s.heavy_min = m->opts.heavy_item_ratings > 0 ? (uint32_t)m->opts.heavy_item_ratings : 32768u;
-    s.n_train = R; s.n_pr = P;
+    s.n_train = R;
+    s.heavy_min = heavy_min_for(m);
+    s.rounded_decay_min = rounded_decay_min_for(m);
+    s.n_pr = P;
     s.day_range = dr;
     s.gbias = (float)(rsum / (double)R);
     m->h_user_cnt.assign(tr.user_cnts, tr.user_cnts + U);

@@ -126,3 +126,44 @@ def test_ycache_rebuild_is_bitwise_at_the_edges_of_its_row_groups(f):
     for n in ("ycache", "ycache_bias"):
         a = np.asarray(g.get_param(n), np.float32).ravel()
         assert np.array_equal(a.view(np.uint32), np.asarray(o.get_param(n), np.float32).ravel().view(np.uint32)), n
+
+
+def counted_items(counts, n_users, seed):
+    """Items with exactly these numbers of training ratings, users' ratings on
+    few days so that several frequency bins meet in an item's rounds."""
+    rng = np.random.default_rng(seed)
+    u = np.concatenate([rng.choice(n_users, size=n, replace=False) for n in counts])
+    i = np.repeat(np.arange(len(counts)), counts)
+    o = np.lexsort((i, u))
+    u, i = u[o], i[o]
+    d = 100 + 40 * (u % 7) + rng.integers(0, 1 + u % 5, size=len(u)) * 3
+    tr = Dataset.from_ratings(u, i, rng.integers(1, 6, len(u)), d, n_users, len(counts), "items_tr")
+    pu, pi = np.arange(n_users), np.full(n_users, len(counts) - 1)
+    ok = ~np.isin(pu * len(counts) + pi, u * len(counts) + i)
+    pr = Dataset.from_ratings(pu[ok], pi[ok], rng.integers(1, 6, ok.sum()), 100 + 40 * (pu[ok] % 7), n_users,
+                              len(counts), "items_pr")
+    return tr, pr
+
+
+ITEM_COUNTS = [1, 2, 3, 5, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 95, 96, 97, 128, 161]
+
+
+@pytest.mark.parametrize("heavy", [1, 40, 100000])
+@pytest.mark.parametrize("f", [0, 20, 40, 96, 128, 160, 224, 256])
+def test_item_stratum_at_the_edges_of_its_rounds_and_pairs(f, heavy):
+    """Items of one rating up to a few rounds of 32, all in rounds (heavy = 1),
+    some, or all by one warp; strong item, bin and frequency updates and decays,
+    so that a wrong weight inside a round shows."""
+    tr, pr = counted_items(ITEM_COUNTS, 200, 5)
+    cfg = run_lm(f, 2, n_time_bins=48).replace(lr_ti=0.002, lr_ibf=0.003, lr_iqf=0.004, reg_iqf=0.05, reg_i=0.05,
+                                               sigma_u=0.1, sigma_i=0.1, sigma_iqf=0.1)
+    check_epochs(tr, pr, cfg, heavy_item_ratings=heavy)
+
+
+@pytest.mark.parametrize("f,bins", [(20, 64), (60, 12), (100, 16), (250, 64)])
+def test_item_stratum_with_the_per_day_rows_and_many_bins(f, bins):
+    """The per-day rows in the rounds' user rows; tables of up to 64 frequency
+    bins beside the widest rows."""
+    tr, pr = counted_items(ITEM_COUNTS, 200, 6)
+    check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30, low_memory=False).replace(n_freq_bins=bins, lr_iqf=0.004),
+                 epochs=1)
