@@ -7,22 +7,6 @@ namespace tsvd {
 // a - 1 for a row's decay factor a = 1 - x, or for that factor rounded to FP32.
 __device__ __forceinline__ float row_decay(float x, bool rounded) { return rounded ? (1.0f - x) - 1.0f : -x; }
 
-// Four tables of 36 floats: a_i^n, a_f^n, a_i^n - 1, a_f^n - 1 for n = 0 .. N. The
-// rounded factors' powers are products in FP32, as those items have had them.
-template <int N>
-__device__ __forceinline__ void decay_powers(float* pow, const EpochParams& p, bool rounded) {
-    const float d_i = row_decay(p.lr_i * p.reg_i, rounded), d_f = row_decay(p.lr_iqf * p.reg_iqf, rounded);
-    float x = 0.0f, y = 0.0f;  // a^n - 1 = (a^(n-1) - 1) a + (a - 1)
-    for (int e = 0; e <= N; ++e) {
-        pow[e] = 1.0f + x;
-        pow[36 + e] = 1.0f + y;
-        pow[72 + e] = x;
-        pow[108 + e] = y;
-        x = rounded ? __fmul_rn(1.0f + x, 1.0f + d_i) - 1.0f : fmaf(x, d_i, x) + d_i;
-        y = rounded ? __fmul_rn(1.0f + y, 1.0f + d_f) - 1.0f : fmaf(y, d_f, y) + d_f;
-    }
-}
-
 // An item's biases, spread over a warp.
 struct ItemState {
     float ib, bt0, bt1, bf0, bf1;
@@ -56,6 +40,14 @@ __device__ __forceinline__ void store_item_state(const DeviceState& s, uint32_t 
 // ---------------------------------------------------------------------------
 constexpr int kLightRows = 4;   // ratings in the ring
 constexpr int kLightAhead = 2;  // ratings asked for ahead
+
+// (out of line: the plain chain's loop stays short)
+static __device__ __noinline__ float ordinal_err(const float* thresholds, float score, int y) {
+    float th[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) th[k] = __ldg(thresholds + k);
+    return ordinal_grad(th, score, y);
+}
 
 template <int VPL, bool BF>
 __device__ __forceinline__ void item_pairs(const DeviceState& s, const EpochParams& p, const Bf16Copies& bf, uint32_t i,

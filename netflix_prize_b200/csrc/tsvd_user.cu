@@ -265,268 +265,6 @@ void launch_user(tsvd_model* m, const DeviceState& s, const EpochParams& p, cons
     m->launches++;
 }
 
-// ---------------------------------------------------------------------------
-// With the per-day terms (low_memory = false): one rating at a time. Each run of
-// equal dates gets its su_day from yfeat_day (the run's training items, then the
-// day's pr items, src/tsvdx4p.rs:500-527), the ratings add ufeat_day and su_day to
-// p_u(t), ufeat_day is trained (:604-611), and at the run's end its error sum over
-// sqrt(day count) goes to every item of the run as a yfeat_day delta (:614-622).
-//
-// A run is a rating or two, so what it starts with decides the chain: its
-// ufeat_day row and its first yfeat_day row are asked for while the run before it
-// is trained (the two runs' days differ, so the row is not about to change), its
-// length comes from the chunk's records in registers, and the item rows come
-// through the ring. 6 M ratings, f = 60: 17.9 ms when each of these was waited for
-// in turn, DAYMS now.
-// ---------------------------------------------------------------------------
-constexpr int day_ctas(int vpl) { return vpl >= 7 ? 3 : vpl >= 5 ? 4 : vpl >= 3 ? 5 : 7; }
-
-// Fixed-point accumulation of a per-day NSVD1 delta row (red.global.add.u64).
-template <int VPL>
-__device__ __forceinline__ void dyd_add(unsigned long long* row, int lane, const float (&x)[VPL]) {
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-        const long long q = __double2ll_rn((double)x[v] * kDydScale);
-        atomicAdd(row + Row<VPL>::elem(lane, v), (unsigned long long)q);
-    }
-}
-
-template <int VPL>
-__global__ void __launch_bounds__(kUThreads, day_ctas(VPL)) k_user_days(DeviceState s, EpochParams p,
-                                                                        const uint32_t* __restrict__ order,
-                                                                        uint32_t n_work) {
-    using V = Vec<VPL>;
-    extern __shared__ __align__(16) float smem[];
-    const int lane = threadIdx.x & 31;
-    const uint32_t Fs = s.Fs, T = s.T, NF = s.NF;
-    float* ring = smem + (threadIdx.x >> 5) * kRingRows * 2 * Fs;
-    const bool ordinal = s.raw != nullptr;
-    for (;;) {
-        uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(&s.counters[0], 1u);
-        k = __shfl_sync(kFull, k, 0);
-        if (k >= n_work) break;
-        const uint32_t u = order[k];
-        const uint64_t start = s.user_off[u], end = s.user_off[u + 1];
-        if (start == end) continue;
-        const uint64_t ps = s.pr_off[u], pe = s.pr_off[u + 1];
-        const uint64_t total = (end - start) + (p.full_su ? (pe - ps) : 0);
-        const float norm = sqrtf((float)total);
-        V su;
-        float sub;
-        if (p.use_ycache) {
-            su.load_cg(s.ycache + (size_t)u * Fs, lane);
-            sub = __ldcg(s.ycache_bias + u);
-        } else {
-            su.zero();
-            sub = 0.0f;
-            const Rec* rr = s.rec + start;
-            const uint32_t* pp = s.pr_item + ps;
-            sum_rows<VPL, false>(s.yfeat, nullptr, s.ybias, Fs, end - start,
-                                 [&](uint64_t q) { return rec_id(__ldg(&rr[q].key)); }, lane, su, sub);
-            sum_rows<VPL, false>(s.yfeat, nullptr, s.ybias, Fs, p.full_su ? pe - ps : 0,
-                                 [&](uint64_t q) { return __ldg(pp + q); }, lane, su, sub);
-            su.divide(norm);
-            sub = sub / norm;
-            su.store_cg(s.ycache + (size_t)u * Fs, lane);
-            if (lane == 0) s.ycache_bias[u] = sub;
-        }
-        V pu, p2, seq;
-        pu.load_cg(s.ufeat + (size_t)u * Fs, lane);
-        p2.load_cg(s.ufeat2 + (size_t)u * Fs, lane);
-        seq.zero();
-        float ub = __ldcg(s.ubias + u), al = __ldcg(s.alpha_u + u), cuu = __ldcg(s.cu + u);
-        float bb0 = lane < (int)T ? __ldcg(s.but_bin + (size_t)u * T + lane) : 0.0f;
-        float bb1 = lane + 32 < (int)T ? __ldcg(s.but_bin + (size_t)u * T + 32 + lane) : 0.0f;
-        float sum_err = 0.0f;
-        // the current run of equal dates, and the next one's first rows
-        V sud, seqd, pud, sn, pn;
-        float norm_day = 1.0f;
-        uint64_t run0 = 0, run1 = 0;
-
-        auto chunk_rec = [&](uint64_t base) { return load_rec(s.rec + min(base + lane, end - 1)); };
-        Rec ahead = chunk_rec(start);
-        // rating j of the chunk whose keys are `keys`: its item's q and q^f row
-        auto ask = [&](uint32_t keys, uint32_t j) {
-            const uint32_t key = __shfl_sync(kFull, keys, j);
-            float* slot = ring + (j % kRingRows) * 2 * Fs;
-            row_cp_async<VPL>(slot, s.ifeat + (size_t)rec_id(key) * Fs, lane);
-            row_cp_async<VPL>(slot + Fs, s.ifeat_freq + ((size_t)rec_id(key) * NF + rec_fbin(key)) * Fs, lane);
-            cp_async_commit();
-        };
-        auto ask_run = [&](uint32_t key, uint32_t ud) {
-            if (p.has_ud && ud < s.n_ud) pn.load_cg(s.ufeat_day + (size_t)ud * Fs, lane);
-            else pn.zero();
-            sn.load_nc(s.yfeat_day + (size_t)rec_id(key) * Fs, lane);
-        };
-#pragma unroll 1
-        for (int q = 0; q < kAheadRows; ++q) ask(ahead.key, q);
-        ask_run(__shfl_sync(kFull, ahead.key, 0), __shfl_sync(kFull, ahead.ud, 0));
-        for (uint64_t base = start; base < end; base += 32) {
-            const uint32_t cnt = (uint32_t)(end - base < 32 ? end - base : 32);
-            const Rec r = ahead;
-            ahead = chunk_rec(base + 32);
-            const uint32_t i = rec_id(r.key), tb = rec_tbin(r.key);
-            const bool hud = r.ud < s.n_ud;
-            const float bi = __ldg(s.ibias + i) + __ldg(s.bit_bin + (size_t)i * T + tb) +
-                             __ldg(s.ibias_freq + (size_t)i * NF + rec_fbin(r.key));
-            const float ct = hud ? __ldg(s.cut + r.ud) : 0.0f;
-            const uint32_t pr_day = p.full_su && hud ? __ldg(s.ud_pr_cnt + r.ud) : 0u;
-            // the day's bias, kept current for every rating of the chunk
-            float bud = hud ? __ldcg(s.ubias_day + r.ud) : 0.0f;
-            // lanes whose rating ends a run (the chunk's last: by the next chunk's first)
-            uint32_t un = __shfl_down_sync(kFull, r.ud, 1);
-            const uint32_t u_next = __shfl_sync(kFull, ahead.ud, 0);
-            if (lane == 31) un = u_next;
-            const unsigned ends = __ballot_sync(kFull, un != r.ud || base + lane + 1 >= end);
-#pragma unroll 1
-            for (uint32_t j = 0; j < cnt; ++j) {
-                {
-                    const bool here = j + kAheadRows < 32;
-                    ask(here ? r.key : ahead.key, (j + kAheadRows) & 31u);
-                }
-                const uint64_t t = base + j;
-                const uint32_t uj = __shfl_sync(kFull, r.ud, j), kj = __shfl_sync(kFull, r.key, j);
-                const bool hj = uj < s.n_ud;
-                if (t == start || t > run1) {
-                    // a new run of equal dates (day_ranges, src/tx.rs:92-104)
-                    const unsigned later = ends & ~((1u << j) - 1u);
-                    run1 = later ? base + __ffs((int)later) - 1 : base + 31;
-                    if (!later)
-                        while (run1 + 1 < end && __ldg(&s.rec[run1 + 1].ud) == uj) ++run1;
-                    run0 = t;
-                    pud = pn;
-                    sud = sn;
-                    seqd.zero();
-                    const uint32_t pc = __shfl_sync(kFull, pr_day, j);
-                    const float day_cnt = (float)(uint32_t)(run1 - t + 1) + (float)pc;
-                    float none = 0.0f;
-                    if (run1 > t)
-                        sum_rows<VPL, false>(s.yfeat_day, nullptr, nullptr, Fs, run1 - t,
-                                             [&](uint64_t q) { return rec_id(__ldg(&s.rec[t + 1 + q].key)); }, lane, sud,
-                                             none);
-                    if (pc) {
-                        const uint32_t* list = s.ud_list_item + s.ud_list_off[uj];
-                        sum_rows<VPL, false>(s.yfeat_day, nullptr, nullptr, Fs, pc,
-                                             [&](uint64_t q) { return __ldg(list + q); }, lane, sud, none);
-                    }
-                    norm_day = sqrtf(day_cnt);
-                    if (day_cnt != 1.0f) sud.divide(norm_day);
-                    const uint64_t nr = run1 + 1;
-                    if (nr < end) {
-                        const uint32_t at = (uint32_t)(nr - base);
-                        if (at < 64) {
-                            const uint32_t nk = __shfl_sync(kFull, at < 32 ? r.key : ahead.key, at & 31);
-                            ask_run(nk, __shfl_sync(kFull, at < 32 ? r.ud : ahead.ud, at & 31));
-                        } else {
-                            const Rec n = load_rec(s.rec + nr);
-                            ask_run(n.key, n.ud);
-                        }
-                    }
-                }
-                cp_async_wait<kAheadRows>();
-                V qe;
-                {
-                    V f;
-                    const float* slot = ring + (j % kRingRows) * 2 * Fs;
-                    qe.load(slot, lane);
-                    f.load(slot + Fs, lane);
-                    qe.add(f);  // q_i + q^f_{i,fb}
-                }
-                const float dv = __shfl_sync(kFull, r.dev, j);
-                float dot;
-                {
-                    V x = su;
-                    x.add(pu);
-                    x.fma(dv, p2);
-                    x.add(pud);
-                    x.add(sud);
-                    dot = warp_sum(qe.dot(x));
-                }
-                const uint32_t tj = rec_tbin(kj);
-                const float but = __shfl_sync(kFull, tj < 32 ? bb0 : bb1, tj & 31);
-                const float bi_t = __shfl_sync(kFull, bi, j);
-                const float bu_t = ub + but + al * dv + __shfl_sync(kFull, bud, j) + sub;
-                const float score = s.gbias + bu_t + bi_t * (cuu + __shfl_sync(kFull, ct, j)) + dot;
-                const float target = __shfl_sync(kFull, r.res, j);
-                const float err = ordinal ? ordinal_err(s.thresholds, score, (int)target) : score - target;
-                ub -= p.lr_ub * err;
-                {
-                    const float nb = but - p.lr_tu * err;
-                    if (lane == (int)(tj & 31)) {
-                        if (tj < 32) bb0 = nb;
-                        else bb1 = nb;
-                    }
-                }
-                al -= p.lr_ta * err * dv;
-                bud -= hud && uj == r.ud ? p.lr_ubd * err : 0.0f;
-                cuu -= p.lr_cu * (err * bi_t + p.reg_cu * (cuu - 1.0f));
-                sum_err += err;
-                seq.fma(err, qe);
-                seqd.fma(err, qe);
-                // x - lr (g + reg x), the change rounded into the row once
-                {
-                    V x = pu;
-                    x.scale(-p.lr_u * p.reg_u);
-                    x.fma(-p.lr_u * err, qe);
-                    pu.add(x);
-                    x = p2;
-                    x.scale(-p.lr_u2 * p.reg_u2);
-                    x.fma(-p.lr_u2 * (err * dv), qe);
-                    p2.add(x);
-                    if (p.has_ud && hj) {
-                        x = pud;
-                        x.scale(-p.lr_ud * p.reg_ud);
-                        x.fma(-p.lr_ud * err, qe);
-                        pud.add(x);
-                    }
-                }
-                if (t == run1) {
-                    // end of the run: ufeat_day back, and the run's yfeat_day delta to
-                    // each of its items
-                    if (p.has_ud && hj) pud.store_cg(s.ufeat_day + (size_t)uj * Fs, lane);
-                    seqd.divide(norm_day);
-                    float gd[VPL];
-                    seqd.to(gd);
-                    dyd_add<VPL>(s.dyd_fix + (size_t)rec_id(kj) * Fs, lane, gd);
-                    for (uint64_t q = run0; q < run1; ++q)
-                        dyd_add<VPL>(s.dyd_fix + (size_t)rec_id(__ldg(&s.rec[q].key)) * Fs, lane, gd);
-                }
-            }
-            // the chunk's day biases (ratings of one day hold the same value)
-            if (hud) __stcg(s.ubias_day + r.ud, bud);
-            __syncwarp();
-        }
-        cp_async_wait<0>();
-        pu.store_cg(s.ufeat + (size_t)u * Fs, lane);
-        p2.store_cg(s.ufeat2 + (size_t)u * Fs, lane);
-        if (lane == 0) {
-            s.ubias[u] = ub;
-            s.alpha_u[u] = al;
-            s.cu[u] = cuu;
-        }
-        if (lane < (int)T) s.but_bin[(size_t)u * T + lane] = bb0;
-        if (lane + 32 < (int)T) s.but_bin[(size_t)u * T + 32 + lane] = bb1;
-        seq.divide(norm);
-        seq.store_cg(s.g_user + (size_t)u * Fs, lane);
-        if (lane == 0) s.e_user[u] = sum_err / norm;
-    }
-}
-
-template <int VPL>
-void launch_days(tsvd_model* m, const DeviceState& s, const EpochParams& p, const uint32_t* work, uint32_t n) {
-    auto kern = k_user_days<VPL>;
-    const size_t smem = (size_t)(kUThreads / 32) * kRingRows * 2 * s.Fs * sizeof(float);
-    int dev = 0, sms = 0, per_sm = 0;
-    TSVD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    TSVD_CUDA(cudaGetDevice(&dev));
-    TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    TSVD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kUThreads, smem));
-    kern<<<(unsigned)(sms * std::max(per_sm, 1)), kUThreads, smem, m->stream>>>(s, p, work, n);
-    TSVD_CUDA(cudaGetLastError());
-    m->launches++;
-}
-
 }  // namespace
 
 void launch_user_stratum(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf,
@@ -537,10 +275,6 @@ void launch_user_stratum(tsvd_model* m, const DeviceState& s, const EpochParams&
     } else {
         TSVD_DISPATCH(vpl, (launch_user<V, false>(m, s, p, bf, work, n)));
     }
-}
-
-void launch_user_days(tsvd_model* m, const DeviceState& s, const EpochParams& p, const uint32_t* work, uint32_t n) {
-    TSVD_DISPATCH((int)(s.Fs / 32), launch_days<V>(m, s, p, work, n));
 }
 
 }  // namespace tsvd
