@@ -600,19 +600,7 @@ __global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_roun
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t Fs = s.Fs, NF = s.NF, T = s.T;
     ItemCtx c{s, p, bf, smem, item_smem(Fs, NF, CW), 0, 0, 0, row_pitch(Fs), nullptr, nullptr, nullptr, nullptr, s.raw != nullptr};
-    if (threadIdx.x < 2) {  // the powers, and those of the rounded factors
-        const float d_i = row_decay(p.lr_i * p.reg_i, threadIdx.x == 1), d_f = row_decay(p.lr_iqf * p.reg_iqf, threadIdx.x == 1);
-        float* pow = smem + c.L.pow + threadIdx.x * 144;
-        float x = 0.0f, y = 0.0f;  // a^n - 1 = (a^(n-1) - 1) a + (a - 1)
-        for (int e = 0; e <= kRound; ++e) {
-            pow[e] = 1.0f + x;
-            pow[36 + e] = 1.0f + y;
-            pow[72 + e] = x;
-            pow[108 + e] = y;
-            x = fmaf(x, d_i, x) + d_i;
-            y = fmaf(y, d_f, y) + d_f;
-        }
-    }
+    if (threadIdx.x < 2) decay_powers<kRound>(smem + c.L.pow + threadIdx.x * 144, p, threadIdx.x == 1);
     // the zero columns of an odd width
     if constexpr (VPL > 1 && (VPL & 1)) {
         const uint32_t P = row_pitch(Fs);

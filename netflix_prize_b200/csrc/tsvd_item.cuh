@@ -4,8 +4,37 @@
 
 namespace tsvd {
 
-// a - 1 for a row's decay factor a = 1 - x, or for that factor rounded to FP32.
-__device__ __forceinline__ float row_decay(float x, bool rounded) { return rounded ? (1.0f - x) - 1.0f : -x; }
+// a - 1 for a row's decay factor a = 1 - lr reg, or for that factor rounded to FP32
+// (once: the product is not rounded before it).
+__device__ __forceinline__ float row_decay(float lr, float reg, bool rounded) {
+    return rounded ? __fmaf_rn(-lr, reg, 1.0f) - 1.0f : -(lr * reg);
+}
+
+// Four tables of 36 floats: a_i^n, a_f^n, a_i^n - 1, a_f^n - 1 for n = 0 .. N. The
+// rounded factors' powers are products in FP32, as those items have had them.
+template <int N>
+__device__ __forceinline__ void decay_powers(float* pow, const EpochParams& p, bool rounded) {
+    const float d_i = row_decay(p.lr_i, p.reg_i, rounded), d_f = row_decay(p.lr_iqf, p.reg_iqf, rounded);
+    float x = 0.0f, y = 0.0f;  // a^n - 1 = (a^(n-1) - 1) a + (a - 1)
+    for (int e = 0; e <= N; ++e) {
+        pow[e] = 1.0f + x;
+        pow[36 + e] = 1.0f + y;
+        pow[72 + e] = x;
+        pow[108 + e] = y;
+        x = rounded ? __fmul_rn(1.0f + x, 1.0f + d_i) - 1.0f : fmaf(x, d_i, x) + d_i;
+        y = rounded ? __fmul_rn(1.0f + y, 1.0f + d_f) - 1.0f : fmaf(y, d_f, y) + d_f;
+    }
+}
+
+// The per-rating a - 1 whose 32nd power is that table's: what a chain of single
+// ratings applies to an item with the rounded factors.
+__device__ __forceinline__ float rounded_step(float d) {
+    float x = 1.0f;
+    for (int e = 0; e < 32; ++e) x = __fmul_rn(x, 1.0f + d);
+    double r = x;
+    for (int e = 0; e < 5; ++e) r = sqrt(r);
+    return (float)(r - 1.0);
+}
 
 // An item's biases, spread over a warp.
 struct ItemState {
@@ -57,7 +86,7 @@ __device__ __forceinline__ void item_pairs(const DeviceState& s, const EpochPara
     const uint64_t start = s.item_off[i], end = s.item_off[i + 1];
     const bool ordinal = s.raw != nullptr;
     const bool rounded = end - start >= s.rounded_decay_min;
-    const float da = row_decay(p.lr_i * p.reg_i, rounded), df = row_decay(p.lr_iqf * p.reg_iqf, rounded);
+    const float di = row_decay(p.lr_i, p.reg_i, rounded), da = rounded ? rounded_step(di) : di, df = row_decay(p.lr_iqf, p.reg_iqf, rounded);
     const float a1 = 1.0f + da, f1 = 1.0f + df;
     const float da2 = fmaf(da, da, 2.0f * da), df2 = fmaf(df, df, 2.0f * df);
     V q;

@@ -247,19 +247,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
     float* sv = smem + L.sv;
     float4* ap = reinterpret_cast<float4*>(smem + L.ap);
     float* sst = smem + L.st;
-    if (threadIdx.x < 2) {  // the powers, and those of the rounded factors
-        const float d_i = row_decay(p.lr_i * p.reg_i, threadIdx.x == 1), d_f = row_decay(p.lr_iqf * p.reg_iqf, threadIdx.x == 1);
-        float* pow = smem + L.pw + threadIdx.x * 144;
-        float x = 0.0f, y = 0.0f;  // a^n - 1 = (a^(n-1) - 1) a + (a - 1)
-        for (int e = 0; e <= kRound; ++e) {
-            pow[e] = 1.0f + x;
-            pow[36 + e] = 1.0f + y;
-            pow[72 + e] = x;
-            pow[108 + e] = y;
-            x = fmaf(x, d_i, x) + d_i;
-            y = fmaf(y, d_f, y) + d_f;
-        }
-    }
+    if (threadIdx.x < 2) decay_powers<kRound>(smem + L.pw + threadIdx.x * 144, p, threadIdx.x == 1);
     const float gb = s.gbias;
     for (;;) {
         if (threadIdx.x == 0) sh_k = atomicAdd(&s.counters[2], 1u);

@@ -178,6 +178,15 @@ std::vector<uint32_t> heaviest_first(const C* cnt, uint32_t n) {
     return out;
 }
 
+// A row's decay by x - lr reg x is added as (a - 1) x, a = 1 - lr reg, which keeps
+// lr reg's own digits. Items of at least this many ratings multiply by a rounded to
+// FP32 instead (for q^f rows, lr reg = 3.5e-8 becomes 6.0e-8): a model trained on
+// from a saved state, or compared with one, keeps the rows it has had.
+uint32_t rounded_decay_min_for(const tsvd_model* m) {
+    if (!m->cfg.low_memory || m->cfg.has_ordinal_head) return 0xffffffffu;
+    return m->opts.heavy_item_ratings > 0 ? (uint32_t)m->opts.heavy_item_ratings : 32768u;
+}
+
 // Heavy items take a CTA each, the others a warp each: a rating then costs the
 // GPU less, but its chain is longer. The line is where a light item's chain is
 // about as long as the pass, in shares of the ratings an SM gets: rows up to 128
@@ -189,16 +198,10 @@ uint32_t heavy_min_for(const tsvd_model* m) {
     int sms = 0;
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
     const uint64_t share = m->d.n_train / ((m->d.Fs > 128 ? 20 : 4) * (uint64_t)sms);
-    return (uint32_t)std::min<uint64_t>(0x7fffffffu, std::max<uint64_t>(64, share));
-}
-
-// A row's decay by x - lr reg x is added as (a - 1) x, a = 1 - lr reg, which keeps
-// lr reg's own digits. Items of at least this many ratings multiply by a rounded to
-// FP32 instead (for q^f rows, lr reg = 3.5e-8 becomes 6.0e-8): a model trained on
-// from a saved state, or compared with one, keeps the rows it has had.
-uint32_t rounded_decay_min_for(const tsvd_model* m) {
-    if (!m->cfg.low_memory || m->cfg.has_ordinal_head) return 0xffffffffu;
-    return m->opts.heavy_item_ratings > 0 ? (uint32_t)m->opts.heavy_item_ratings : 32768u;
+    // (rows above 128 columns: items with the rounded factors all take a CTA, where
+    // those are applied)
+    const uint64_t most = m->d.Fs > 128 ? std::min(0x7fffffffu, rounded_decay_min_for(m)) : 0x7fffffffu;
+    return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(64, share));
 }
 
 void setup_model(tsvd_model* m, const tsvd_dataset_view& tr, const tsvd_dataset_view& pr) {
