@@ -222,6 +222,15 @@ __device__ __forceinline__ void load_thresholds(const DeviceState& s, float (&th
     for (int k = 0; k < 4; ++k) th[k] = s.raw ? __ldg(s.thresholds + k) : 0.0f;
 }
 
+// The head's gradient at a score, out of line where the plain chain's loop should
+// stay short.
+static __device__ __noinline__ float ordinal_err(const float* thresholds, float score, int y) {
+    float th[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) th[k] = __ldg(thresholds + k);
+    return ordinal_grad(th, score, y);
+}
+
 // User-side scalars of one by-item rating: bu_t and cu_t (src/tsvdx4p.rs:690-708).
 __device__ __forceinline__ void user_scalars(const DeviceState& s, const Rec& r, float& bu_t, float& cu_t) {
     const uint32_t u = rec_id(r.key), tb = rec_tbin(r.key);
@@ -235,6 +244,9 @@ __device__ __forceinline__ void user_scalars(const DeviceState& s, const Rec& r,
 // (tsvd_user.cu): the n users of `work`, item rows from qe0.
 void launch_user_stratum(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf,
                          const uint32_t* work, uint32_t n);
+
+// With the per-day terms (low_memory = false), rows up to 256 columns.
+void launch_user_days(tsvd_model* m, const DeviceState& s, const EpochParams& p, const uint32_t* work, uint32_t n);
 
 // The item stratum of rows up to 256 columns (tsvd_item.cu): the items of
 // s.item_work, heaviest first.

@@ -70,14 +70,6 @@ __device__ __forceinline__ void store_item_state(const DeviceState& s, uint32_t 
 constexpr int kLightRows = 4;   // ratings in the ring
 constexpr int kLightAhead = 2;  // ratings asked for ahead
 
-// (out of line: the plain chain's loop stays short)
-static __device__ __noinline__ float ordinal_err(const float* thresholds, float score, int y) {
-    float th[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) th[k] = __ldg(thresholds + k);
-    return ordinal_grad(th, score, y);
-}
-
 template <int VPL, bool BF>
 __device__ __forceinline__ void item_pairs(const DeviceState& s, const EpochParams& p, const Bf16Copies& bf, uint32_t i,
                                            int lane, float* ring) {

@@ -57,240 +57,10 @@ __global__ void k_make_qe0(const float* __restrict__ ifeat, const float* __restr
 void make_qe0(tsvd_model* m, bool bf16);
 
 
-// su gather with 8 rows in flight, in the reference's order.
-template <int VPL, class ItemOf>
-__device__ __forceinline__ void gather_y_ro(const DeviceState& s, uint64_t n, ItemOf item_of, int lane,
-                                            float (&su)[VPL], float& sub) {
-    constexpr int B = 8;
-    for (uint64_t base = 0; base < n; base += 32) {
-        const uint32_t cnt = (uint32_t)(n - base < 32 ? n - base : 32);
-        const uint32_t mine = lane < (int)cnt ? item_of(base + lane) : 0u;
-        for (uint32_t j = 0; j < cnt; j += B) {
-            float y[B][VPL], yb[B];
-#pragma unroll
-            for (int q = 0; q < B; ++q) {
-                const uint32_t it = __shfl_sync(kFull, mine, j + q < cnt ? j + q : cnt - 1);
-                Row<VPL>::load_nc(s.yfeat + (size_t)it * s.Fs, lane, y[q]);
-                yb[q] = __ldg(s.ybias + it);
-            }
-#pragma unroll
-            for (int q = 0; q < B; ++q) {
-                if (j + q < cnt) {
-#pragma unroll
-                    for (int v = 0; v < VPL; ++v) su[v] += y[q][v];
-                    sub += yb[q];
-                }
-            }
-        }
-    }
-}
-
 // err of a rating: score - residual, or with the ordinal head the gradient of
 // -log P(y) in the score (src/tx.rs:963-972); `target` is then the raw rating.
 __device__ __forceinline__ float rating_err(const DeviceState& s, const float (&th)[4], float score, float target) {
     return s.raw ? ordinal_grad(th, score, (int)target) : score - target;
-}
-
-// Fixed-point accumulation of a per-day NSVD1 delta row (red.global.add.u64).
-template <int VPL>
-__device__ __forceinline__ void dyd_add(unsigned long long* row, int lane, const float (&x)[VPL]) {
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-        const long long q = __double2ll_rn((double)x[v] * kDydScale);
-        atomicAdd(row + Row<VPL>::elem(lane, v), (unsigned long long)q);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// User stratum with the per-day terms (low_memory = false; fit_epoch_user,
-// src/tsvdx4p.rs:390-639; without them tsvd_user.cu). Item tables are read-only
-// here; the item rows of rating j+1 are requested before rating j is used. Each
-// run of equal dates gets its su_day from yfeat_day (the run's training items,
-// then the day's pr items, :500-527), the ratings add ufeat_day and su_day to
-// p_u(t), ufeat_day is trained (:604-611), and at the run's end its error sum
-// over sqrt(day count) goes to every item of the run as a yfeat_day delta
-// (:614-622).
-// ---------------------------------------------------------------------------
-template <int VPL>
-__global__ void __launch_bounds__(kThreads, 2) k_user_strat(DeviceState s, EpochParams p,
-                                                            const uint32_t* __restrict__ order, uint32_t n_work) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t Fs = s.Fs, T = s.T, NF = s.NF;
-    float th[4];
-    load_thresholds(s, th);
-    for (;;) {
-        uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(&s.counters[0], 1u);
-        k = __shfl_sync(kFull, k, 0);
-        if (k >= n_work) break;
-        const uint32_t u = order[k];
-        const uint64_t start = s.user_off[u], end = s.user_off[u + 1];
-        if (start == end) continue;
-        const uint64_t ps = s.pr_off[u], pe = s.pr_off[u + 1];
-        const uint64_t total = (end - start) + (p.full_su ? (pe - ps) : 0);
-        const float norm = sqrtf((float)total);
-
-        // su (src/tsvdx4p.rs:466-491): equals ycache[u] bit for bit when full_su
-        // holds and ycache was rebuilt from the current y.
-        float su[VPL], sub;
-        if (p.use_ycache) {
-            Row<VPL>::load_cg(s.ycache + (size_t)u * Fs, lane, su);
-            sub = __ldcg(s.ycache_bias + u);
-        } else {
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) su[v] = 0.0f;
-            sub = 0.0f;
-            const Rec* rr = s.rec + start;
-            gather_y_ro<VPL>(s, end - start, [&](uint64_t q) { return rec_id(__ldg(&rr[q].key)); }, lane, su, sub);
-            if (p.full_su) {
-                const uint32_t* pp = s.pr_item + ps;
-                gather_y_ro<VPL>(s, pe - ps, [&](uint64_t q) { return __ldg(pp + q); }, lane, su, sub);
-            }
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) su[v] = su[v] / norm;
-            sub = sub / norm;
-            Row<VPL>::store(s.ycache + (size_t)u * Fs, lane, su);
-            if (lane == 0) s.ycache_bias[u] = sub;
-        }
-
-        float pu[VPL], p2[VPL], seq[VPL];
-        Row<VPL>::load_cg(s.ufeat + (size_t)u * Fs, lane, pu);
-        Row<VPL>::load_cg(s.ufeat2 + (size_t)u * Fs, lane, p2);
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) seq[v] = 0.0f;
-        float ub = __ldcg(s.ubias + u), al = __ldcg(s.alpha_u + u), cuu = __ldcg(s.cu + u);
-        float bb0 = lane < (int)T ? __ldcg(s.but_bin + (size_t)u * T + lane) : 0.0f;
-        float bb1 = lane + 32 < (int)T ? __ldcg(s.but_bin + (size_t)u * T + 32 + lane) : 0.0f;
-        float sum_err = 0.0f;
-        const float gb = s.gbias;
-        // the current run of equal dates
-        float sud[VPL], seqd[VPL], pud[VPL];
-        float norm_day = 1.0f;
-        uint64_t run0 = 0, run1 = 0;
-
-        for (uint64_t base = start; base < end; base += 32) {
-            const uint32_t cnt = (uint32_t)(end - base < 32 ? end - base : 32);
-            Rec mine{};
-            if (lane < (int)cnt) mine = load_rec(s.rec + base + lane);
-            float qn[VPL], qfn[VPL];
-            auto fetch_item = [&](uint32_t key) {
-                Row<VPL>::load_nc(s.ifeat + (size_t)rec_id(key) * Fs, lane, qn);
-                Row<VPL>::load_nc(s.ifeat_freq + ((size_t)rec_id(key) * NF + rec_fbin(key)) * Fs, lane, qfn);
-            };
-            fetch_item(__shfl_sync(kFull, mine.key, 0));
-            for (uint32_t j = 0; j < cnt; ++j) {
-                const Rec r = shfl_rec(mine, j);
-                const uint32_t i = rec_id(r.key), tb = rec_tbin(r.key);
-                const uint32_t fb = rec_fbin(r.key);
-                const bool hud = r.ud < s.n_ud;
-                const uint64_t t = base + j;
-                if (t == start || t > run1) {
-                    // a new run of equal dates (day_ranges, src/tx.rs:92-104)
-                    run0 = run1 = t;
-                    while (run1 + 1 < end && __ldg(&s.rec[run1 + 1].ud) == r.ud) ++run1;
-#pragma unroll
-                    for (int v = 0; v < VPL; ++v) sud[v] = seqd[v] = 0.0f;
-                    float dummy = 0.0f;
-                    gather_rows8<VPL>(s.yfeat_day, nullptr, Fs, run1 - run0 + 1,
-                                      [&](uint64_t q) { return rec_id(__ldg(&s.rec[run0 + q].key)); }, lane, sud,
-                                      dummy);
-                    float day_cnt = (float)(run1 - run0 + 1);
-                    if (p.full_su && hud) {
-                        const uint64_t off = s.ud_list_off[r.ud];
-                        const uint32_t pc = s.ud_pr_cnt[r.ud];
-                        gather_rows8<VPL>(s.yfeat_day, nullptr, Fs, pc,
-                                          [&](uint64_t q) { return __ldg(s.ud_list_item + off + q); }, lane, sud,
-                                          dummy);
-                        for (uint32_t c = 0; c < pc; ++c) day_cnt += 1.0f;
-                    }
-                    norm_day = sqrtf(day_cnt);
-#pragma unroll
-                    for (int v = 0; v < VPL; ++v) sud[v] = sud[v] / norm_day;
-                    if (p.has_ud && hud) Row<VPL>::load_cg(s.ufeat_day + (size_t)r.ud * Fs, lane, pud);
-                    else
-#pragma unroll
-                        for (int v = 0; v < VPL; ++v) pud[v] = 0.0f;
-                }
-            
-                float qe[VPL];  // q_i + q^f_{i,fb}
-#pragma unroll
-                for (int v = 0; v < VPL; ++v) {
-                    qe[v] = qn[v] + qfn[v];
-                }
-                if (j + 1 < cnt) fetch_item(__shfl_sync(kFull, mine.key, j + 1));
-                const float ib = __ldg(s.ibias + i);
-                const float bit = __ldg(s.bit_bin + (size_t)i * T + tb);
-                const float ibf = __ldg(s.ibias_freq + (size_t)i * NF + fb);
-                float bud = 0.0f;
-                if (lane == 0 && hud) bud = s.ubias_day[r.ud];
-                bud = __shfl_sync(kFull, bud, 0);
-                const float ct = hud ? __ldg(s.cut + r.ud) : 0.0f;
-                const float but = __shfl_sync(kFull, tb < 32 ? bb0 : bb1, tb & 31);
-                const float dv = r.dev;
-                const float bu_t = ub + but + al * dv + bud + sub;
-                const float bi_t = ib + bit + ibf;
-                const float cu_t = cuu + ct;
-                float part = 0.0f;
-#pragma unroll
-                for (int v = 0; v < VPL; ++v) {
-                    float pev = (pu[v] + su[v]) + dv * p2[v];
-                    if (p.has_ud && hud) pev += pud[v];
-                    pev += sud[v];
-                
-                    part += qe[v] * pev;
-                }
-                const float dot = warp_sum(part);
-                const float err = rating_err(s, th, gb + bu_t + bi_t * cu_t + dot, r.res);
-                ub -= p.lr_ub * err;
-                {
-                    const float nb = but - p.lr_tu * err;
-                    if (lane == (int)(tb & 31)) {
-                        if (tb < 32) bb0 = nb;
-                        else bb1 = nb;
-                    }
-                }
-                al -= p.lr_ta * err * dv;
-                if (lane == 0 && hud) s.ubias_day[r.ud] = bud - p.lr_ubd * err;
-                cuu -= p.lr_cu * (err * bi_t + p.reg_cu * (cuu - 1.0f));
-                sum_err += err;
-#pragma unroll
-                for (int v = 0; v < VPL; ++v) {
-                    const float pk = pu[v], p2k = p2[v];
-                    seq[v] += err * qe[v];
-                    pu[v] = pk - p.lr_u * (err * qe[v] + p.reg_u * pk);
-                    p2[v] = p2k - p.lr_u2 * (err * qe[v] * dv + p.reg_u2 * p2k);
-                    seqd[v] += err * qe[v];
-                    if (p.has_ud && hud) pud[v] = pud[v] - p.lr_ud * (err * qe[v] + p.reg_ud * pud[v]);
-                
-                }
-                if (t == run1) {
-                    // end of the run: ufeat_day back, and the run's yfeat_day
-                    // delta to each of its items (src/tsvdx4p.rs:614-622)
-                    if (p.has_ud && hud) Row<VPL>::store(s.ufeat_day + (size_t)r.ud * Fs, lane, pud);
-                    float gd[VPL];
-#pragma unroll
-                    for (int v = 0; v < VPL; ++v) gd[v] = seqd[v] / norm_day;
-                    for (uint64_t q2 = run0; q2 <= run1; ++q2)
-                        dyd_add<VPL>(s.dyd_fix + (size_t)rec_id(__ldg(&s.rec[q2].key)) * Fs, lane, gd);
-                }
-            
-            }
-        }
-        Row<VPL>::store(s.ufeat + (size_t)u * Fs, lane, pu);
-        Row<VPL>::store(s.ufeat2 + (size_t)u * Fs, lane, p2);
-        if (lane == 0) {
-            s.ubias[u] = ub;
-            s.alpha_u[u] = al;
-            s.cu[u] = cuu;
-        }
-        if (lane < (int)T) s.but_bin[(size_t)u * T + lane] = bb0;
-        if (lane + 32 < (int)T) s.but_bin[(size_t)u * T + 32 + lane] = bb1;
-        float g[VPL];
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) g[v] = seq[v] / norm;
-        Row<VPL>::store(s.g_user + (size_t)u * Fs, lane, g);
-        if (lane == 0) s.e_user[u] = sum_err / norm;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -855,10 +625,7 @@ void strat_launch(tsvd_model* m, const EpochParams& p, const Bf16Copies& bf) {
     {
         ProfScope ps(m, "user_pass_stratified");
         if constexpr (DAY) {
-            unsigned g = persistent_grid(k_user_strat<VPL>, 0);
-            k_user_strat<VPL><<<g, kThreads, 0, m->stream>>>(s, p, s.user_work, s.n_users);
-            TSVD_CUDA(cudaGetLastError());
-            m->launches++;
+            launch_user_days(m, s, p, s.user_work, s.n_users);
         } else {
             launch_user_stratum(m, s, p, bf, s.user_work, s.n_users);
         }
@@ -909,10 +676,7 @@ __global__ void k_reset_users(DeviceState s, const uint32_t* __restrict__ users,
 template <int VPL>
 void foldin_launch(tsvd_model* m, const EpochParams& p, const uint32_t* d_users, uint32_t n) {
     if (m->d.dyd_fix) {
-        unsigned g = persistent_grid(k_user_strat<VPL>, 0);
-        k_user_strat<VPL><<<g, kThreads, 0, m->stream>>>(m->d, p, d_users, n);
-        TSVD_CUDA(cudaGetLastError());
-        m->launches++;
+        launch_user_days(m, m->d, p, d_users, n);
     } else {
         make_qe0(m, false);
         launch_user_stratum(m, m->d, p, Bf16Copies{}, d_users, n);
@@ -939,10 +703,7 @@ void shard_user_launch(tsvd_model* m, const EpochParams& p, const uint32_t* work
             m->launches++;
         } else {
             if constexpr (DAY) {
-                unsigned g = persistent_grid(k_user_strat<VPL>, 0);
-                k_user_strat<VPL><<<g, kThreads, 0, m->stream>>>(s, p, work, n);
-                TSVD_CUDA(cudaGetLastError());
-                m->launches++;
+                launch_user_days(m, s, p, work, n);
             } else {
                 launch_user_stratum(m, s, p, Bf16Copies{}, work, n);
             }

@@ -167,3 +167,41 @@ def test_item_stratum_with_the_per_day_rows_and_many_bins(f, bins):
     tr, pr = counted_items(ITEM_COUNTS, 200, 6)
     check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30, low_memory=False).replace(n_freq_bins=bins, lr_iqf=0.004),
                  epochs=1)
+
+
+def patterned_days(n_items, seed):
+    """Users whose days follow patterns, in item order: each day once, days that
+    come back one to four ratings later, runs of two and more (one over three
+    chunks of 32), lone ratings beside runs; query pairs on every fourth day."""
+    rng = np.random.default_rng(seed)
+    u, i, d, pu, pi, pd = [], [], [], [], [], []
+    patterns = ["abcdefgh", "ab", "abc", "abac", "abcd", "aab", "abb", "aabb", "abcca", "a" * 70 + "b"]
+    k = 0
+    for p in patterns:
+        for n in (1, 2, 3, 31, 32, 33, 34, 65, 97):
+            items = np.sort(rng.choice(n_items, size=n + 2, replace=False))
+            q = rng.permutation(n + 2)
+            days = [5 * k % 1400 + ord(p[j % len(p)]) + (3 * j if p == "abcdefgh" else 0) for j in range(n)]
+            u += [k] * n
+            i += list(items[np.sort(q[:n])])
+            d += days
+            if k % 4 == 0:
+                pu += [k] * 2
+                pi += list(items[q[n:]])
+                pd += [days[0], days[-1]]
+            k += 1
+    tr = Dataset.from_ratings(u, i, rng.integers(1, 6, len(u)), d, k, n_items, "days_tr")
+    o = np.lexsort((np.array(pu), np.array(pi)))
+    pr = Dataset.from_ratings(np.array(pu)[o], np.array(pi)[o], rng.integers(1, 6, len(pu)), np.array(pd)[o], k,
+                              n_items, "days_pr")
+    return tr, pr
+
+
+@pytest.mark.parametrize("f,full_su,lr_ud", [(20, True, 0.005), (60, True, 0.005), (60, False, 0.005), (60, True, 0.0),
+                                             (90, True, 0.005), (128, True, 0.005), (190, True, 0.005),
+                                             (256, True, 0.005)])
+def test_user_stratum_with_the_per_day_rows(f, full_su, lr_ud):
+    """Pairs of lone ratings, ufeat_day rows handed on between ratings of one day,
+    and runs of equal dates; two epochs, so that the day rows are not zero."""
+    tr, pr = patterned_days(150, 7)
+    check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30, low_memory=False).replace(full_su=full_su, lr_ud=lr_ud))
