@@ -248,6 +248,12 @@ void launch_user_stratum(tsvd_model* m, const DeviceState& s, const EpochParams&
 // With the per-day terms (low_memory = false), rows up to 256 columns.
 void launch_user_days(tsvd_model* m, const DeviceState& s, const EpochParams& p, const uint32_t* work, uint32_t n);
 
+// Rows of more than 256 columns, by a block per user or item (tsvd_wide.cu), where
+// wide_pairs_fit(Fs).
+bool wide_pairs_fit(uint32_t Fs);
+void launch_user_wide_pairs(tsvd_model* m, const DeviceState& s, const EpochParams& p, const uint32_t* work, uint32_t n);
+void launch_item_wide_pairs(tsvd_model* m, const DeviceState& s, const EpochParams& p);
+
 // The item stratum of rows up to 256 columns (tsvd_item.cu): the items of
 // s.item_work, heaviest first.
 void launch_item_stratum(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf);

@@ -336,7 +336,8 @@ __global__ void __launch_bounds__(kThreads) k_y_apply_sums(DeviceState s, EpochP
 }
 
 // ---------------------------------------------------------------------------
-// n_feat > 256 (the tsvdx4 400lm ... 4800lm jobs, tsvdx4p up to 16000): rows
+// Rows above 2,048 columns (tsvd_wide.cu has those of more than 256; the tsvdx4 jobs
+// go up to 4800 factors, tsvdx4p up to 16000): rows
 // of Fs = 256 k columns. A warp's unit keeps its own rows in global memory
 // (they are private to it, and each lane reads back only what it wrote) and
 // takes each rating in two passes over 256-column slices: the dot product,
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(kThreads) k_user_strat_wide(DeviceState s, Epo
     }
 }
 
-// Item stratum for wide rows: one warp per item, the item's q and q^f rows in
+// Item stratum for rows above 2,048 columns: one warp per item, the item's q and q^f rows in
 // global memory, every item on the one-warp chain.
 __global__ void __launch_bounds__(kThreads) k_item_wide(DeviceState s, EpochParams p) {
     using R8 = Row<kWV>;
@@ -567,15 +568,33 @@ __global__ void __launch_bounds__(kThreads) k_item_wide(DeviceState s, EpochPara
     }
 }
 
+// The wide strata's launches.
+void launch_user_wide(tsvd_model* m, const EpochParams& p, const uint32_t* work, uint32_t n) {
+    if (wide_pairs_fit(m->d.Fs)) {
+        launch_user_wide_pairs(m, m->d, p, work, n);
+        return;
+    }
+    k_user_strat_wide<<<persistent_grid(k_user_strat_wide, 0), kThreads, 0, m->stream>>>(m->d, p, work, n);
+    TSVD_CUDA(cudaGetLastError());
+    m->launches++;
+}
+
+void launch_item_wide(tsvd_model* m, const DeviceState& s, const EpochParams& p) {
+    if (wide_pairs_fit(s.Fs)) {
+        launch_item_wide_pairs(m, s, p);
+        return;
+    }
+    k_item_wide<<<persistent_grid(k_item_wide, 0), kThreads, 0, m->stream>>>(s, p);
+    TSVD_CUDA(cudaGetLastError());
+    m->launches++;
+}
+
 void strat_launch_wide(tsvd_model* m, const EpochParams& p) {
     const DeviceState& s = m->d;
     make_qe0(m, false);
     {
         ProfScope ps(m, "user_pass_stratified");
-        unsigned g = persistent_grid(k_user_strat_wide, 0);
-        k_user_strat_wide<<<g, kThreads, 0, m->stream>>>(s, p, s.user_work, s.n_users);
-        TSVD_CUDA(cudaGetLastError());
-        m->launches++;
+        launch_user_wide(m, p, s.user_work, s.n_users);
     }
     {
         ProfScope ps(m, "y_apply");
@@ -587,10 +606,7 @@ void strat_launch_wide(tsvd_model* m, const EpochParams& p) {
     launch_rebuild_ycache(m, s.pyc);
     {
         ProfScope ps(m, "item_pass");
-        unsigned g = persistent_grid(k_item_wide, 0);
-        k_item_wide<<<g, kThreads, 0, m->stream>>>(s, p);
-        TSVD_CUDA(cudaGetLastError());
-        m->launches++;
+        launch_item_wide(m, s, p);
     }
 }
 
@@ -697,10 +713,7 @@ void shard_user_launch(tsvd_model* m, const EpochParams& p, const uint32_t* work
     {
         ProfScope ps(m, "user_pass_stratified");
         if (s.Fs > kSlice) {
-            unsigned g = persistent_grid(k_user_strat_wide, 0);
-            k_user_strat_wide<<<g, kThreads, 0, m->stream>>>(s, p, work, n);
-            TSVD_CUDA(cudaGetLastError());
-            m->launches++;
+            launch_user_wide(m, p, work, n);
         } else {
             if constexpr (DAY) {
                 launch_user_days(m, s, p, work, n);
@@ -723,10 +736,7 @@ void shard_item_launch(tsvd_model* m, const EpochParams& p, const uint32_t* work
     s.n_item_work = n;
     ProfScope ps(m, "item_pass");
     if (s.Fs > kSlice) {
-        unsigned g = persistent_grid(k_item_wide, 0);
-        k_item_wide<<<g, kThreads, 0, m->stream>>>(s, p);
-        TSVD_CUDA(cudaGetLastError());
-        m->launches++;
+        launch_item_wide(m, s, p);
     } else {
         launch_item_stratum(m, s, p, Bf16Copies{});
     }

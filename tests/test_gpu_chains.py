@@ -205,3 +205,14 @@ def test_user_stratum_with_the_per_day_rows(f, full_su, lr_ud):
     and runs of equal dates; two epochs, so that the day rows are not zero."""
     tr, pr = patterned_days(150, 7)
     check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30, low_memory=False).replace(full_su=full_su, lr_ud=lr_ud))
+
+
+@pytest.mark.parametrize("f,bins", [(257, 16), (600, 16), (1000, 16), (1100, 16), (1600, 30), (2048, 16), (2100, 16)])
+def test_rows_above_256_columns(f, bins):
+    """A block per unit up to 2,048 columns, with the q^f rows in shared memory (16 or
+    8 ratings in the ring) and in the table; a warp per unit above."""
+    counts = [1, 2, 3, 6, 7, 8, 15, 16, 17, 31, 32, 33, 34, 46, 63, 64, 65, 97, 1, 2]
+    tr, pr = counted_sets(counts, 120, 8)
+    check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30).replace(n_freq_bins=bins, lr_iqf=0.004), epochs=1)
+    tr, pr = counted_items([c for c in ITEM_COUNTS if c <= 150], 150, 9)
+    check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30).replace(n_freq_bins=bins, lr_iqf=0.004), epochs=1)
