@@ -1,7 +1,7 @@
 // Batched prediction: TxModel::predict (src/tx.rs:713-724 via factor_parts
 // :303-339), predict_subscores (:651-711), and the FP64 sum of squared errors
-// behind calc_rmse (src/lib.rs:659-672). One warp per row; the SSE is reduced
-// in a fixed order (per-warp sums, per-block tree, then one block over the
+// behind calc_rmse (src/lib.rs:659-672). A warp per row, or per group of rows; the
+// SSE is reduced in a fixed order (per-lane sums, per-warp and per-block trees, then one block over the
 // block partials), so repeated calls are bitwise identical.
 #include <algorithm>
 #include <mutex>
@@ -101,58 +101,167 @@ __device__ __forceinline__ bool row_in_range(const DeviceState& s, uint32_t u, u
     return u < s.n_users && i < s.n_items;
 }
 
+// The scores of a warp's rows, one row per lane (want: the lane has one). The lanes
+// look up their rows' scalars side by side (the search for the user-day is a chain of
+// six to eight loads, and a warp per row waits for all of it before the last feature
+// row), then the warp takes the feature rows of two rows at a time.
 template <int VPL>
-__global__ void __launch_bounds__(kThreads) k_predict(DeviceState s, PredParams pp, const int32_t* __restrict__ u,
-                                                      const int32_t* __restrict__ it, const int16_t* __restrict__ d,
-                                                      const float* __restrict__ offset, uint64_t n,
-                                                      float* __restrict__ out, int subscores) {
+__device__ __forceinline__ float score_rows(const DeviceState& s, const PredParams& pp, bool want, uint32_t u, uint32_t i,
+                                            int16_t day, int lane) {
+    const uint32_t Fs = s.Fs, T = s.T, NF = s.NF;
+    uint32_t idx = 0xffffffffu, qf_at = 0;
+    float dv = 0.0f, bp = 0.0f, dot = 0.0f;
+    if (want) {
+        const uint32_t b = time_bin(day, s.day_range, T);
+        dv = dev_of(day, s.tu_mean[u], pp.beta);
+        idx = ud_index(s, u, day);
+        const bool has = idx != 0xffffffffu;
+        const uint32_t f = has ? freq_bin(s.ud_cnt[idx], NF) : 0u;
+        const float bu_day = has ? s.ubias_day[idx] : 0.0f;
+        const float ubu = s.ubias[u], but = s.but_bin[(size_t)u * T + b], al = s.alpha_u[u], ycb = s.ycache_bias[u];
+        const float ibi = s.ibias[i], bit = s.bit_bin[(size_t)i * T + b], ibf = s.ibias_freq[(size_t)i * NF + f];
+        const float bu_t = ubu + but + al * dv + bu_day + ycb;
+        const float bi_t = ibi + bit + ibf;
+        const float cu_t = s.cu[u] + (has ? s.cut[idx] : 0.0f);
+        bp = s.gbias + bu_t + bi_t * cu_t;
+        qf_at = i * NF + f;
+    }
+    unsigned todo = __ballot_sync(kFull, want);
+    while (todo) {
+        int at[2];
+        at[0] = at[1] = __ffs((int)todo) - 1;
+        todo &= todo - 1;
+        const bool two = todo != 0;
+        if (two) {
+            at[1] = __ffs((int)todo) - 1;
+            todo &= todo - 1;
+        }
+        uint32_t uj[2], ij[2], fj[2], dj[2];
+        float vj[2], part[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            uj[k] = __shfl_sync(kFull, u, at[k]);
+            ij[k] = __shfl_sync(kFull, i, at[k]);
+            fj[k] = __shfl_sync(kFull, qf_at, at[k]);
+            dj[k] = __shfl_sync(kFull, idx, at[k]);
+            vj[k] = __shfl_sync(kFull, dv, at[k]);
+        }
+        for (uint32_t c0 = 0; c0 < Fs; c0 += 32 * VPL) {
+            float pu[2][VPL], p2[2][VPL], su[2][VPL], q[2][VPL], qf[2][VPL];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (k == 1 && !two) break;
+                Row<VPL>::load_nc(s.ufeat + (size_t)uj[k] * Fs + c0, lane, pu[k]);
+                Row<VPL>::load_nc(s.ufeat2 + (size_t)uj[k] * Fs + c0, lane, p2[k]);
+                Row<VPL>::load_nc(s.ycache + (size_t)uj[k] * Fs + c0, lane, su[k]);
+                Row<VPL>::load_nc(s.ifeat + (size_t)ij[k] * Fs + c0, lane, q[k]);
+                Row<VPL>::load_nc(s.ifeat_freq + (size_t)fj[k] * Fs + c0, lane, qf[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (k == 1 && !two) break;
+                float pe[VPL];
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) pe[v] = (pu[k][v] + su[k][v]) + vj[k] * p2[k][v];
+                if (!pp.low_memory && dj[k] != 0xffffffffu) {
+                    float pd[VPL], sd[VPL];
+                    Row<VPL>::load_nc(s.ufeat_day + (size_t)dj[k] * Fs + c0, lane, pd);
+                    Row<VPL>::load_nc(s.ycache_day + (size_t)dj[k] * Fs + c0, lane, sd);
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) {
+                        pe[v] += pd[v];
+                        pe[v] += sd[v];
+                    }
+                }
+#pragma unroll
+                for (int v = 0; v < VPL; ++v) part[k] += pe[v] * (q[k][v] + qf[k][v]);
+            }
+        }
+        const float d0 = warp_sum(part[0]), d1 = warp_sum(part[1]);
+        if (lane == at[0]) dot = d0;
+        if (two && lane == at[1]) dot = d1;
+    }
+    return want ? finish_score(s, pp, bp, dot) : 0.0f;
+}
+
+// Rows per warp and pass: as many as leave every warp of the grid four passes. Few
+// rows are bound by one row's chain of loads, which a warp per row spreads best; with
+// four passes each the warps are full either way.
+uint32_t rows_per_warp(uint64_t n, uint64_t warps) {
+    uint32_t g = 1;
+    while (g < 32 && n / (2 * g) >= 4 * warps) g *= 2;
+    return g;
+}
+
+// Bound by the reads of the user rows (3 KB a row at f = 256, from HBM where rows come
+// in item order): 4.2 M rows of 480,189 users 6.0 -> 2.2 ms, 12.9 GB in 2.0 at the
+// rate of a plain copy.
+template <int VPL>
+__global__ void __launch_bounds__(kThreads, 2) k_predict_rows(DeviceState s, PredParams pp, const int32_t* __restrict__ u,
+                                                              const int32_t* __restrict__ it,
+                                                              const int16_t* __restrict__ d,
+                                                              const float* __restrict__ offset, uint64_t n, uint32_t per,
+                                                              float* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t step = (uint64_t)gridDim.x * kWarps * per;
+    for (uint64_t r0 = (blockIdx.x * (uint64_t)kWarps + (threadIdx.x >> 5)) * per; r0 < n; r0 += step) {
+        const uint64_t r = r0 + lane;
+        const bool mine = lane < (int)per && r < n;
+        const uint32_t ur = mine ? (uint32_t)u[r] : 0u, ir = mine ? (uint32_t)it[r] : 0u;
+        const bool in = mine && row_in_range(s, ur, ir);
+        float x = score_rows<VPL>(s, pp, in, ur, ir, in ? d[r] : (int16_t)0, lane);
+        if (in && offset) x += offset[r];
+        // an index outside the model's tables: no table is read, the row's output is
+        // NaN (device entry points cannot raise per row)
+        if (mine) out[r] = in ? x : __int_as_float(0x7fc00000);
+    }
+}
+
+template <int VPL>
+__global__ void __launch_bounds__(kThreads) k_subscores(DeviceState s, PredParams pp, const int32_t* __restrict__ u,
+                                                        const int32_t* __restrict__ it, const int16_t* __restrict__ d,
+                                                        uint64_t n, float* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t)gridDim.x * kWarps;
     for (uint64_t r = blockIdx.x * (uint64_t)kWarps + (threadIdx.x >> 5); r < n; r += warps) {
-        float bp = 0.0f, dot = 0.0f, sub[3];
+        float bp, dot, sub[3];
         const uint32_t ur = (uint32_t)u[r], ir = (uint32_t)it[r];
-        if (!row_in_range(s, ur, ir)) {
-            // an index outside the model's tables: no table is read, the row's
-            // outputs are NaN (device entry points cannot raise per row)
-            if (lane == 0) {
-                if (subscores) out[3 * r] = out[3 * r + 1] = out[3 * r + 2] = __int_as_float(0x7fc00000);
-                else out[r] = __int_as_float(0x7fc00000);
-            }
-            continue;
-        }
-        predict_row<VPL>(s, pp, ur, ir, d[r], lane, bp, dot, subscores ? sub : nullptr);
+        if (row_in_range(s, ur, ir)) predict_row<VPL>(s, pp, ur, ir, d[r], lane, bp, dot, sub);
+        else sub[0] = sub[1] = sub[2] = __int_as_float(0x7fc00000);  // as in k_predict_rows
         if (lane == 0) {
-            if (subscores) {
-                out[3 * r] = sub[0];
-                out[3 * r + 1] = sub[1];
-                out[3 * r + 2] = sub[2];
-            } else {
-                const float score = finish_score(s, pp, bp, dot);
-                out[r] = offset ? score + offset[r] : score;
-            }
+            out[3 * r] = sub[0];
+            out[3 * r + 1] = sub[1];
+            out[3 * r + 2] = sub[2];
         }
     }
 }
 
 template <int VPL>
-__global__ void __launch_bounds__(kThreads) k_sse(DeviceState s, PredParams pp, const int32_t* __restrict__ u,
+__global__ void __launch_bounds__(kThreads, 2) k_sse(DeviceState s, PredParams pp, const int32_t* __restrict__ u,
                                                   const int32_t* __restrict__ it, const int16_t* __restrict__ d,
                                                   const float* __restrict__ target, const int8_t* __restrict__ is_test,
-                                                  uint64_t n, double* __restrict__ part_sse,
+                                                  uint64_t n, uint32_t per, double* __restrict__ part_sse,
                                                   double* __restrict__ part_cnt) {
     __shared__ double ssh[kWarps], csh[kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t warps = (uint64_t)gridDim.x * kWarps;
     double sse = 0.0, cnt = 0.0;
-    for (uint64_t r = blockIdx.x * (uint64_t)kWarps + warp; r < n; r += warps) {
-        if (is_test && is_test[r] != 0) continue;
-        if (!row_in_range(s, (uint32_t)u[r], (uint32_t)it[r])) continue;  // the host checked the rows
-        float bp = 0.0f, dot = 0.0f;
-        predict_row<VPL>(s, pp, (uint32_t)u[r], (uint32_t)it[r], d[r], lane, bp, dot, nullptr);
-        const float e = finish_score(s, pp, bp, dot) - target[r];
-        const double ed = (double)e;
-        sse += ed * ed;
-        cnt += 1.0;
+    for (uint64_t r0 = (blockIdx.x * (uint64_t)kWarps + warp) * per; r0 < n; r0 += warps * per) {
+        const uint64_t r = r0 + lane;
+        bool in = lane < (int)per && r < n && !(is_test && is_test[r] != 0);
+        const uint32_t ur = in ? (uint32_t)u[r] : 0u, ir = in ? (uint32_t)it[r] : 0u;
+        in = in && row_in_range(s, ur, ir);  // the host checked the rows
+        const float x = score_rows<VPL>(s, pp, in, ur, ir, in ? d[r] : (int16_t)0, lane);
+        if (in) {
+            const double ed = (double)(x - target[r]);
+            sse += ed * ed;
+            cnt += 1.0;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        sse += __shfl_xor_sync(kFull, sse, o);
+        cnt += __shfl_xor_sync(kFull, cnt, o);
     }
     if (lane == 0) {
         ssh[warp] = sse;
@@ -205,8 +314,14 @@ void predict_device(const tsvd_model* mc, const int32_t* u, const int32_t* i, co
     ProfScope ps(m, subscores ? "predict_subscores" : "predict");
     PredParams pp{m->cfg.beta, m->cfg.low_memory, m->cfg.has_ordinal_head};
     const int vpl = (int)std::min<uint32_t>(m->d.Fs / 32, 8);
-    unsigned grid = (unsigned)std::min<uint64_t>((n + kWarps - 1) / kWarps, 148ull * 16);
-    TSVD_DISPATCH(vpl, (k_predict<V><<<grid, kThreads, 0, m->stream>>>(m->d, pp, u, i, day, offset, n, out, subscores)));
+    if (subscores) {
+        const unsigned grid = (unsigned)std::min<uint64_t>((n + kWarps - 1) / kWarps, 148ull * 16);
+        TSVD_DISPATCH(vpl, (k_subscores<V><<<grid, kThreads, 0, m->stream>>>(m->d, pp, u, i, day, n, out)));
+    } else {
+        const uint32_t per = rows_per_warp(n, 148ull * 2 * kWarps);
+        const unsigned grid = (unsigned)std::min<uint64_t>((n + kWarps * per - 1) / (kWarps * per), 148ull * 4);
+        TSVD_DISPATCH(vpl, (k_predict_rows<V><<<grid, kThreads, 0, m->stream>>>(m->d, pp, u, i, day, offset, n, per, out)));
+    }
     TSVD_CUDA(cudaGetLastError());
     m->launches++;
 }
@@ -223,8 +338,9 @@ void sse_device(const tsvd_model* mc, const int32_t* u, const int32_t* i, const 
     double* psse = m->m_scratch.as<double>();
     double* pcnt = psse + kSseBlocks;
     double* fin = pcnt + kSseBlocks;
-    TSVD_DISPATCH(vpl, (k_sse<V><<<kSseBlocks, kThreads, 0, m->stream>>>(m->d, pp, u, i, day, target, is_test, n, psse,
-                                                                         pcnt)));
+    const uint32_t per = rows_per_warp(n, kSseBlocks * kWarps);
+    TSVD_DISPATCH(vpl, (k_sse<V><<<kSseBlocks, kThreads, 0, m->stream>>>(m->d, pp, u, i, day, target, is_test, n, per,
+                                                                         psse, pcnt)));
     k_sse_final<<<1, 32, 0, m->stream>>>(psse, pcnt, kSseBlocks, fin);
     TSVD_CUDA(cudaGetLastError());
     m->launches += 2;

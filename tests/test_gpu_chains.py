@@ -5,8 +5,11 @@ Tolerance: a parameter is a sum of at most a few hundred updates of at most
 |lr x| ~ 1e-2 each, in FP32 in both, in another order; 2e-5 absolute is the
 bound every other parity test of one epoch holds.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
+import torch
 
 from netflix_prize_b200.abi import PREC_FP32
 from netflix_prize_b200.config import OrdinalHeadConfig, run_lm
@@ -216,3 +219,42 @@ def test_rows_above_256_columns(f, bins):
     check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30).replace(n_freq_bins=bins, lr_iqf=0.004), epochs=1)
     tr, pr = counted_items([c for c in ITEM_COUNTS if c <= 150], 150, 9)
     check_epochs(tr, pr, run_lm(f, 2, n_time_bins=30).replace(n_freq_bins=bins, lr_iqf=0.004), epochs=1)
+
+
+@pytest.mark.parametrize("f,low_memory", [(20, True), (60, False), (96, True), (256, True), (256, False), (400, True)])
+def test_many_rows_score_as_few(f, low_memory):
+    """Predictions by groups of 2 to 32 rows a warp are, bit for bit, those of a warp
+    per row, rows outside the tables (NaN) among them; the RMSE is that of these
+    scores (sums of n squares in FP64: relative error below n 2^-53 = 4e-11)."""
+    tr, pr = counted_items(ITEM_COUNTS, 200, 10)
+    g = TxModel(tr, MaskedDataset(pr), run_lm(f, 1, n_time_bins=30, low_memory=low_memory))
+    g.fit_epoch(tr, pr, 1)
+    rng = np.random.default_rng(11)
+    n = 303150
+    u, i = rng.integers(0, 200, n), np.sort(rng.integers(0, len(ITEM_COUNTS), n))
+    d = rng.choice(np.concatenate([tr.dates, rng.integers(0, 2000, 50)]), n)
+
+    def scores(sel, v):
+        t = [torch.as_tensor(np.ascontiguousarray(x[sel]), device="cuda", dtype=ty)
+             for x, ty in ((v, torch.int32), (i, torch.int32), (d, torch.int16))]
+        out = torch.empty(len(t[0]), device="cuda")
+        torch.cuda.synchronize()
+        g._check(g._L.tsvd_predict_batch_device(g.h, *[C.c_void_p(x.data_ptr()) for x in t], len(out),
+                                                C.c_void_p(out.data_ptr())))
+        torch.cuda.synchronize()
+        return out.cpu().numpy().view(np.uint32)
+
+    wild = u.copy()
+    wild[rng.integers(0, n, 3000)] = 200
+    wild[rng.integers(0, n, 3000)] = -1
+    few = np.concatenate([scores(slice(a, a + 15000), wild) for a in range(0, n, 15000)])
+    assert np.isnan(few.view(np.float32)).sum() > 5000
+    for m in (18943, 18944, 18977, 75777, n):
+        assert np.array_equal(scores(slice(0, m), wild), few[:m]), m
+    raw = rng.integers(1, 6, n)
+    o = np.lexsort((u, i))
+    u, i, d = u[o], i[o], d[o]
+    held = Dataset.from_ratings(u, i, raw, d, 200, len(ITEM_COUNTS), "held")
+    e = (scores(slice(0, n), u).view(np.float32) - held.residuals.astype(np.float32)).astype(np.float64)
+    want = np.sqrt(np.mean(e * e))
+    assert abs(g.calc_rmse(held) - want) < 1e-10 * want
