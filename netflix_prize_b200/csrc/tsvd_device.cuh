@@ -137,22 +137,14 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf
 
 // d(-log P(Y = y)) / d(score), y in 1..5 (OrdinalHead::grad, src/lib.rs:562-598)
 __device__ __forceinline__ float ordinal_grad(const float (&th)[4], float score, int y) {
-    float f[6], a[6];
-    f[0] = 0.0f;
-    f[5] = 1.0f;
-#pragma unroll
-    for (int k = 1; k < 5; ++k) f[k] = sigmoid_f(th[k - 1] - score);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) a[k] = f[k] * (1.0f - f[k]);
-    float fy = f[1], fy1 = f[0], ay = a[1], ay1 = a[0];
-#pragma unroll
-    for (int k = 2; k <= 5; ++k)
-        if (y == k) {
-            fy = f[k];
-            fy1 = f[k - 1];
-            ay = a[k];
-            ay1 = a[k - 1];
-        }
+    // the two of the four cumulative probabilities that bound P(Y = y) (the chains
+    // wait for this value rating by rating: all four took 7.0 ms of item pass where
+    // these take 6.4, 3 M ratings, f = 20)
+    const float hi = y == 2 ? th[1] : y == 3 ? th[2] : y == 4 ? th[3] : th[0];
+    const float lo = y == 3 ? th[1] : y == 4 ? th[2] : y == 5 ? th[3] : th[0];
+    const float sh = sigmoid_f(hi - score), sl = sigmoid_f(lo - score);
+    const float fy = y == 5 ? 1.0f : sh, fy1 = y >= 2 && y <= 5 ? sl : 0.0f;
+    const float ay = fy * (1.0f - fy), ay1 = fy1 * (1.0f - fy1);
     const float p_y = fmaxf(fy - fy1, 1e-6f);
     return (ay - ay1) / p_y;
 }

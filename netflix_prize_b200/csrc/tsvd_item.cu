@@ -533,12 +533,18 @@ __device__ __forceinline__ void consume(const ItemCtx& c, uint32_t r, int cw, in
         if (lane >= kHalf) err = e1;
     } else {
         const int y = (int)V[vTarget * kRound + lane];
+        // four steps in straight-line code, their entries of M asked for at once (3 M
+        // ratings, f = 20: 6.0 ms against 6.4 one by one)
 #pragma unroll 1
-        for (int k = 0; k < kRound; ++k) {
-            const float mk = k < lane ? M[lane * kMPitch + k] : 0.0f;
-            const float ek = valid ? ordinal_grad(th, x, y) : 0.0f;
-            if (k == lane) err = ek;
-            x = fmaf(-mk, __shfl_sync(kFull, ek, k), x);
+        for (int k0 = 0; k0 < kRound; k0 += 4) {
+            const float4 m4 = *reinterpret_cast<const float4*>(M + lane * kMPitch + k0);
+            const float mk[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float ek = valid ? ordinal_grad(th, x, y) : 0.0f;
+                if (k0 + e == lane) err = ek;
+                x = fmaf(k0 + e < lane ? -mk[e] : 0.0f, __shfl_sync(kFull, ek, k0 + e), x);
+            }
         }
     }
     // the updates' weights, every warp some rows of the table
