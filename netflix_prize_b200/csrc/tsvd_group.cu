@@ -16,9 +16,8 @@
 // as one CUDA graph. A variant's item stratum is bounded by the serial chains
 // of its most-rated items, which hold a few SMs; the other variants' strata
 // fill the rest of the GPU meanwhile. The autotuner picks, per feature width,
-// which items run as whole-CTA tiles (rounds of 32 ratings solved together on
-// the tensor cores) and which run one warp each, by timing candidate
-// thresholds on throwaway copies.
+// which items run as whole-CTA tiles (rounds of 32 ratings solved together) and
+// which run one warp each, by timing candidate thresholds on throwaway copies.
 #include <algorithm>
 #include <chrono>
 #include <cstring>

@@ -629,10 +629,7 @@ void to_bf16(tsvd_model* m, const float* src, uint64_t rows, uint64_t src_stride
 
 // One stratified epoch (Tsvdx4pModel::fit_epoch, src/tsvdx4p.rs:815-822):
 // user stratum, NSVD1 delta sums and apply, ycache (and ycache_day) rebuild,
-// item stratum. The item stratum's whole-block path solves a round's errors
-// as a linear system, which holds for err = score - r only: with the ordinal
-// head, and with the per-day terms (which that path does not stage), every
-// item takes the one-warp chain.
+// item stratum.
 template <int VPL, bool BF, bool BFU, bool DAY>
 void strat_launch(tsvd_model* m, const EpochParams& p, const Bf16Copies& bf) {
     DeviceState s = m->d;
