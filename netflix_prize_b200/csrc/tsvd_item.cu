@@ -607,14 +607,11 @@ __global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_roun
     const uint32_t Fs = s.Fs, NF = s.NF, T = s.T;
     ItemCtx c{s, p, bf, smem, item_smem(Fs, NF, CW), 0, 0, 0, row_pitch(Fs), nullptr, nullptr, nullptr, nullptr, s.raw != nullptr};
     if (threadIdx.x < 2) decay_powers<kRound>(smem + c.L.pow + threadIdx.x * 144, p, threadIdx.x == 1);
-    // the zero columns of an odd width
+    // the zero columns of an odd width (those of q and q^f come with each item: an
+    // update by a weight that is not finite leaves them not zero)
     if constexpr (VPL > 1 && (VPL & 1)) {
         const uint32_t P = row_pitch(Fs);
-        for (uint32_t e = threadIdx.x; e < (3 * kRound + NF) * 32; e += blockDim.x) {
-            const uint32_t row = e / 32;
-            smem[(row < 3 * kRound ? c.L.pe + row * P : c.L.qf + (row - 3 * kRound) * P) + Fs + e % 32] = 0.0f;
-        }
-        if (threadIdx.x < 32) smem[c.L.q + Fs + threadIdx.x] = 0.0f;
+        for (uint32_t e = threadIdx.x; e < 3 * kRound * 32; e += blockDim.x) smem[c.L.pe + e / 32 * P + Fs + e % 32] = 0.0f;
     }
     float th[4];
     load_thresholds(s, th);
@@ -644,16 +641,18 @@ __global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_roun
             float qv[CPL];
 #pragma unroll
             for (int v = 0; v < CPL; ++v) qv[v] = 0.0f;
-            if (here && first) {
+            if (first) {
 #pragma unroll
-                for (int v = 0; v < CPL; ++v) smem[c.L.q + col + v] = qv[v] = __ldcg(s.ifeat + (size_t)i * Fs + col + v);
+                for (int v = 0; v < CPL; ++v)
+                    smem[c.L.q + col + v] = qv[v] = here ? __ldcg(s.ifeat + (size_t)i * Fs + col + v) : 0.0f;
             }
-            if (here && (!two || !first)) {
+            if (!two || !first) {
 #pragma unroll 4
                 for (uint32_t b = 0; b < NF; ++b)
 #pragma unroll
                     for (int v = 0; v < CPL; ++v)
-                        smem[c.L.qf + b * c.pitch + col + v] = __ldcg(s.ifeat_freq + ((size_t)i * NF + b) * Fs + col + v);
+                        smem[c.L.qf + b * c.pitch + col + v] =
+                            here ? __ldcg(s.ifeat_freq + ((size_t)i * NF + b) * Fs + col + v) : 0.0f;
             }
             __syncwarp();
             __syncthreads();
