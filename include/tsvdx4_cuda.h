@@ -151,9 +151,13 @@ typedef struct tsvd_gpu_options {
     int32_t heavy_item_ratings; /* stratified item stratum: items with at least
                                 this many ratings take a whole block (rounds of
                                 32 ratings solved together), the others one
-                                warp each (all of them a block for n_feat above
-                                256); 0 = default: a share of the ratings, set
-                                by the data's size and n_feat                 */
+                                warp each; 0 = default: a share of the ratings,
+                                set by the data's size and n_feat. Speed only.
+                                Not used with the per-day terms and for n_feat
+                                of 257 to 2048 (every item takes a block) and
+                                above (every item takes a warp); at most 32768
+                                for n_feat of 129 to 256 without the ordinal
+                                head                                          */
     int32_t seq_epochs[5];   /* stratified: Tsvdx4pConfig::seq_epochs
                                 (src/tsvdx4p.rs:181-186,815-822): these
                                 1-based epochs run the sequential schedule

@@ -179,12 +179,14 @@ std::vector<uint32_t> heaviest_first(const C* cnt, uint32_t n) {
 }
 
 // A row's decay by x - lr reg x is added as (a - 1) x, a = 1 - lr reg, which keeps
-// lr reg's own digits. Items of at least this many ratings multiply by a rounded to
-// FP32 instead (for q^f rows, lr reg = 3.5e-8 becomes 6.0e-8): a model trained on
-// from a saved state, or compared with one, keeps the rows it has had.
+// lr reg's own digits. In the plain form (rows up to 256 columns) items of at least
+// this many ratings multiply by a rounded to FP32 instead, which is not what x - lr
+// reg x gives: lr reg = 3.5e-8 (the q^f rows' default) becomes 6.0e-8. They have
+// always had that: the exact factor moves a q^f row by 2.5e-8 of itself a rating (1 %
+// an epoch for 476,450 ratings), and a model trained on from a saved state keeps its
+// course. heavy_item_ratings does not move this line.
 uint32_t rounded_decay_min_for(const tsvd_model* m) {
-    if (!m->cfg.low_memory || m->cfg.has_ordinal_head) return 0xffffffffu;
-    return m->opts.heavy_item_ratings > 0 ? (uint32_t)m->opts.heavy_item_ratings : 32768u;
+    return !m->cfg.low_memory || m->cfg.has_ordinal_head ? 0xffffffffu : 32768u;
 }
 
 // Heavy items take a CTA each, the others a warp each: a rating then costs the
@@ -194,14 +196,13 @@ uint32_t rounded_decay_min_for(const tsvd_model* m) {
 // 13.0 at 60,000; wider rows (f = 256) 16.9 ms at a twentieth (8,000), 19.9 at
 // 20,000, and 60.4 at 32,768 of 100 M.
 uint32_t heavy_min_for(const tsvd_model* m) {
-    if (m->opts.heavy_item_ratings > 0) return (uint32_t)m->opts.heavy_item_ratings;
     int sms = 0;
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
     const uint64_t share = m->d.n_train / ((m->d.Fs > 128 ? 20 : 4) * (uint64_t)sms);
-    // (rows above 128 columns: items with the rounded factors all take a CTA, where
-    // those are applied)
+    const uint64_t line = m->opts.heavy_item_ratings > 0 ? (uint64_t)m->opts.heavy_item_ratings : std::max<uint64_t>(64, share);
+    // rows above 128 columns: the one-warp chain there has no rounded factors
     const uint64_t most = m->d.Fs > 128 ? std::min(0x7fffffffu, rounded_decay_min_for(m)) : 0x7fffffffu;
-    return (uint32_t)std::min<uint64_t>(most, std::max<uint64_t>(64, share));
+    return (uint32_t)std::min(most, line);
 }
 
 void setup_model(tsvd_model* m, const tsvd_dataset_view& tr, const tsvd_dataset_view& pr) {

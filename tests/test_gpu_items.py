@@ -51,3 +51,76 @@ def test_a_row_that_is_not_finite_stays_with_its_item(f, low_memory, ordinal):
     for n in ITEM_PARAMS:
         assert np.isfinite(got[0][n]).all(), n
         assert np.array_equal(got[1][n][sms:], got[0][n][sms:]), n
+
+
+def long_items(counts):
+    """Item k is rated by the first counts[k] users, each rating on a day of its own
+    (one frequency bin); a query pair a user."""
+    n = max(counts)
+    u = np.concatenate([np.arange(c) for c in counts])
+    i = np.repeat(np.arange(len(counts)), counts)
+    o = np.lexsort((i, u))
+    u, i = u[o], i[o]
+    tr = Dataset.from_ratings(u, i, 1 + (u * 7 + i * 3) % 5, 100 * (i + 1) + u % 50, n, len(counts) + 1, "long")
+    pr = Dataset.from_ratings(np.arange(n), np.full(n, len(counts)), np.full(n, 3), np.full(n, 900), n, len(counts) + 1,
+                              "long_pr")
+    return tr, pr
+
+
+@pytest.mark.parametrize("f", [32])
+def test_decay_does_not_depend_on_the_block_threshold(f):
+    """Items of 32,768 ratings and more decay by factors rounded to FP32 (5.96e-8 here),
+    shorter ones by the exact ones (3.5e-8), whichever of the two paths takes them.
+
+    Tolerance: an item's row is rounded at most once a rating, half an ulp each way:
+    sqrt(40000) 2^-25 = 6e-6 of the row, four times that for the largest of 32 columns.
+    The other factor would be 5000 x 2.4e-8 = 1.2e-4 off in the shortest item."""
+    counts = [40000, 32767, 5000]
+    tr, pr = long_items(counts)
+    zero = {k: 0.0 for k in ("lr_u", "lr_u2", "lr_ub", "lr_ubd", "lr_y", "lr_yb", "lr_ta", "lr_tu", "lr_cu", "lr_ib",
+                             "lr_ti", "lr_ibf")}
+    cfg = run_lm(f, 1, n_time_bins=30).replace(lr_i=5e-6, reg_i=0.007, lr_iqf=5e-6, reg_iqf=0.007, **zero)
+    rng = np.random.default_rng(4)
+    init = {"ufeat": rng.normal(0, 1 / np.sqrt(f), (max(counts), f)).astype(np.float32),
+            "ifeat": rng.normal(0, 0.3, (4, f)).astype(np.float32),
+            "ifeat_freq": rng.normal(0, 0.3, (4 * cfg.n_freq_bins, f)).astype(np.float32),
+            "yfeat": np.zeros((4, f), np.float32)}
+    lr, reg = float(np.float32(5e-6)), float(np.float32(0.007))
+    rounded = float(np.float32(1.0 - lr * reg))
+    assert abs(rounded - (1.0 - 2.0 ** -24)) < 1e-12
+    want = []
+    for heavy in (0, 1, 4096, 100000):
+        m = TxModel(tr, MaskedDataset(pr), cfg, heavy_item_ratings=heavy)
+        for n, v in init.items():
+            m.set_param(n, v)
+        m.fit_epoch(tr, pr, 1)
+        if not want:
+            p, g = init["ufeat"].astype(np.float64), float(np.asarray(m.get_param("gbias")).ravel()[0])
+            for k, c in enumerate(counts):
+                a = rounded if c >= 32768 else 1.0 - lr * reg
+                q, h = init["ifeat"][k].astype(np.float64), init["ifeat_freq"][k * cfg.n_freq_bins].astype(np.float64)
+                for x, y in zip(p[:c], 1 + (np.arange(c) * 7 + k * 3) % 5):
+                    d = lr * (g + x @ (q + h) - y) * x
+                    q, h = a * q - d, a * h - d
+                want.append((q, h))
+        q, h = m.get_param("ifeat"), m.get_param("ifeat_freq").reshape(4, cfg.n_freq_bins, f)[:, 0]
+        for k in range(3):
+            for got, w in ((q[k], want[k][0]), (h[k], want[k][1])):
+                assert np.max(np.abs(got - w)) < 2.4e-5 * np.max(np.abs(w)), (heavy, k)
+
+
+@pytest.mark.parametrize("f", [32, 160])
+def test_thresholds_that_take_the_same_items_give_the_same_bits(f):
+    """Every item here has more than 4,096 ratings. Above 128 columns items of 32,768
+    ratings take a block at any threshold."""
+    tr, pr = long_items([40000, 32767, 5000])
+    cfg = run_lm(f, 1, n_time_bins=30)
+    for same in ((0, 1, 4096), (32768, 40000, 100000) if f > 128 else (32768, 40000)):
+        got = []
+        for heavy in same:
+            m = TxModel(tr, MaskedDataset(pr), cfg, heavy_item_ratings=heavy)
+            m.fit_epoch(tr, pr, 1)
+            got.append({n: np.asarray(m.get_param(n), np.float32).view(np.uint32) for n in ITEM_PARAMS})
+        for g in got[1:]:
+            for n in ITEM_PARAMS:
+                assert np.array_equal(g[n], got[0][n]), (same, n)
