@@ -151,8 +151,9 @@ typedef struct tsvd_gpu_options {
     int32_t heavy_item_ratings; /* stratified item stratum: items with at least
                                 this many ratings take a whole block (rounds of
                                 32 ratings solved together), the others one
-                                warp each; 0 = default: a share of the ratings,
-                                set by the data's size and n_feat. Speed only.
+                                warp each; 0 (or INT32_MAX) = default: a share
+                                of the ratings, set by the data's size and
+                                n_feat. Speed only.
                                 Not used with the per-day terms and for n_feat
                                 of 257 to 2048 (every item takes a block) and
                                 above (every item takes a warp); at most 32768
@@ -338,9 +339,12 @@ int tsvd_group_fit_epoch(tsvd_group* g, uint64_t epoch);
 int tsvd_group_set_graphs(tsvd_group* g, int32_t enabled);
 /* Device time of the last group epoch (CUDA events around the launch). */
 int tsvd_group_last_epoch_ms(const tsvd_group* g, double* out);
-/* Picks the Hogwild prefetch depth (2..4 staged ratings) per feature width by
+/* Hogwild: picks the prefetch depth (2..4 staged ratings) per feature width by
  * timing each candidate on throwaway parameter copies over the units of the
- * sample_users heaviest users; chosen_stages (n_models ints) may be NULL. */
+ * sample_users heaviest users. Stratified: picks the item stratum's threshold
+ * per feature width, among the default and constants that are faster; the value
+ * is a heavy_item_ratings that gives a single model the same results (INT32_MAX:
+ * the default). chosen_stages (n_models ints) may be NULL. */
 int tsvd_group_autotune(tsvd_group* g, uint32_t sample_users, int32_t* chosen_stages);
 const char* tsvd_group_last_error(const tsvd_group* g);
 

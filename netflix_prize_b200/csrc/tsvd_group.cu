@@ -214,11 +214,16 @@ void strat_group_epoch(tsvd_group* g, uint64_t epoch) {
 
 // Per feature width, the whole-CTA threshold of the item stratum that runs a
 // stratified epoch fastest (CUDA events, best of two after a warm-up), timed
-// on a throwaway variant with fresh parameters.
+// on a throwaway variant with fresh parameters: the one that the data's size and
+// the width set (below 2.4 M ratings finer than all the others), or a constant that
+// is faster by more than two runs of one differ. A TxModel created with the reported
+// value as heavy_item_ratings has the same threshold and the same results.
 void strat_autotune(tsvd_group* g, int32_t* chosen) {
     tsvd_model* m0 = g->models[0];
-    const uint32_t cands[] = {0xffffffffu, 65536u, 32768u, 16384u, 8192u, 4096u};
-    std::vector<uint32_t> best_for(9, m0->d.heavy_min);
+    // 0x7fffffff: the size's own (as 0, for a model created with it)
+    const int32_t cands[] = {0x7fffffff, 65536, 32768, 16384, 8192, 4096};
+    constexpr double kFaster = 0.98;
+    int32_t best_for[9] = {};
     for (uint32_t vpl = 1; vpl <= 8; ++vpl) {
         const tsvd_model* rep = nullptr;
         for (auto* m : g->models)
@@ -230,8 +235,9 @@ void strat_autotune(tsvd_group* g, int32_t* chosen) {
         std::unique_ptr<tsvd_model, void (*)(tsvd_model*)> tmp(make_variant(m0, rep->cfg), tsvd_destroy);
         const uint64_t ep = rep->cfg.reset_u_epoch == 1000000 ? 1000001 : 1000000;
         double best = 1e30;
-        for (uint32_t thr : cands) {
-            tmp->d.heavy_min = thr;
+        for (int32_t thr : cands) {
+            tmp->opts.heavy_item_ratings = thr;
+            tmp->d.heavy_min = tsvd::heavy_min_for(tmp.get());
             double t_best = 1e30;
             for (int rep_i = 0; rep_i < 3; ++rep_i) {
                 cudaEvent_t e0, e1;
@@ -247,7 +253,7 @@ void strat_autotune(tsvd_group* g, int32_t* chosen) {
                 cudaEventDestroy(e1);
                 if (rep_i > 0) t_best = std::min<double>(t_best, ms);  // the first run warms up
             }
-            if (t_best < best) {
+            if (t_best < kFaster * best) {
                 best = t_best;
                 best_for[vpl] = thr;
             }
@@ -255,8 +261,9 @@ void strat_autotune(tsvd_group* g, int32_t* chosen) {
     }
     for (size_t k = 0; k < g->models.size(); ++k) {
         tsvd_model* m = g->models[k];
-        m->d.heavy_min = best_for[m->d.Fs / 32];
-        if (chosen) chosen[k] = (int32_t)std::min<uint32_t>(m->d.heavy_min, 0x7fffffffu);
+        m->opts.heavy_item_ratings = best_for[m->d.Fs / 32];
+        m->d.heavy_min = tsvd::heavy_min_for(m);
+        if (chosen) chosen[k] = m->opts.heavy_item_ratings;
     }
     drop_graph(g);  // the captured graph baked in the old thresholds
 }

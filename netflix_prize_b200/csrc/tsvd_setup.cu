@@ -199,7 +199,8 @@ uint32_t heavy_min_for(const tsvd_model* m) {
     int sms = 0;
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));
     const uint64_t share = m->d.n_train / ((m->d.Fs > 128 ? 20 : 4) * (uint64_t)sms);
-    const uint64_t line = m->opts.heavy_item_ratings > 0 ? (uint64_t)m->opts.heavy_item_ratings : std::max<uint64_t>(64, share);
+    const int32_t given = m->opts.heavy_item_ratings;  // (the largest: as 0)
+    const uint64_t line = given > 0 && given < 0x7fffffff ? (uint64_t)given : std::max<uint64_t>(64, share);
     // rows above 128 columns: the one-warp chain there has no rounded factors
     const uint64_t most = m->d.Fs > 128 ? std::min(0x7fffffffu, rounded_decay_min_for(m)) : 0x7fffffffu;
     return (uint32_t)std::min(most, line);
