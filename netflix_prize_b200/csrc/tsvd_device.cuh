@@ -11,6 +11,19 @@ namespace tsvd {
 
 constexpr unsigned kFull = 0xffffffffu;
 
+// The most dynamic shared memory a kernel is launched with: of the 227 KB a block can
+// have, all but 1 KB for static arrays.
+constexpr size_t kMaxDynSmem = 226 * 1024;
+
+// Lets a kernel be launched with up to that. Never a launch's own size: models of
+// several shapes share a kernel, and a thread that trains one would lower the limit
+// between another's call and its launch.
+template <class K>
+void allow_dyn_smem(K kernel, size_t smem) {
+    if (smem > kMaxDynSmem) throw Error(TSVD_ERR_UNSUPPORTED, "a block would need " + std::to_string(smem) + " bytes of shared memory");
+    TSVD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem));
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);

@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_rebuild_ycache(DeviceState s, c
 template <int VPL>
 void launch_hog_pass(tsvd_model* m, const EpochParams& p, const uint32_t* order) {
     const size_t smem = (size_t)kWarps * hog_ring_floats(kStages, m->d.Fs) * sizeof(float);
-    TSVD_CUDA(cudaFuncSetAttribute(k_hog_pass<VPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(k_hog_pass<VPL>, smem);
     unsigned g = persistent_grid(k_hog_pass<VPL>, smem);
     k_hog_pass<VPL><<<g, kThreads, smem, m->stream>>>(m->d, p, order, m->d.n_users);
     TSVD_CUDA(cudaGetLastError());
@@ -466,7 +466,7 @@ void launch_rebuild(tsvd_model* m, const __nv_bfloat16* ybf, float* pyc) {
 void launch_hog_batched(cudaStream_t st, const DeviceState* d_states, const EpochParams* d_params,
                         const uint32_t* d_units, uint32_t n_units, uint32_t ring_floats, uint32_t* d_counter) {
     const size_t smem = (size_t)kWarps * ring_floats * sizeof(float);
-    TSVD_CUDA(cudaFuncSetAttribute(k_hog_batched, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(k_hog_batched, smem);
     unsigned g = persistent_grid(k_hog_batched, smem);
     k_hog_batched<<<g, kThreads, smem, st>>>(d_states, d_params, d_units, n_units, ring_floats, d_counter);
     TSVD_CUDA(cudaGetLastError());

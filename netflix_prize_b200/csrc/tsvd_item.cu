@@ -763,7 +763,7 @@ void launch_item(tsvd_model* m, const DeviceState& s, const EpochParams& p, cons
     auto kern = k_item_rounds<VPL, MODE>;
     const size_t smem = std::max<size_t>(item_smem(s.Fs, s.NF, consumers(VPL)).total,
                                          light_smem(item_threads(VPL) / 32, s.Fs)) * sizeof(float);
-    TSVD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(kern, smem);
     int dev = 0, sms = 0, per_sm = 0;
     TSVD_CUDA(cudaGetDevice(&dev));
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

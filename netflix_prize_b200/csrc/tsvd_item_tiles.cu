@@ -663,7 +663,7 @@ template <int VPL, bool BF>
 void launch_tiles(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf) {
     auto kern = k_item_pass<VPL, BF>;
     const size_t smem = (size_t)item_smem(s.Fs, s.NF).total * sizeof(float);
-    TSVD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(kern, smem);
     int dev = 0, sms = 0;
     TSVD_CUDA(cudaGetDevice(&dev));
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -264,7 +264,7 @@ void launch_user(tsvd_model* m, const DeviceState& s, const EpochParams& p, cons
     auto kern = k_user_pairs<VPL, ORD>;
     const size_t smem = (size_t)(kUThreads / 32) * kRingRows * s.Fs * sizeof(float);
     int dev = 0, sms = 0, per_sm = 0;
-    TSVD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(kern, smem);
     TSVD_CUDA(cudaGetDevice(&dev));
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TSVD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kUThreads, smem));
@@ -600,7 +600,7 @@ void launch_days(tsvd_model* m, const DeviceState& s, const EpochParams& p, cons
     auto kern = k_user_day_pairs<VPL>;
     const size_t smem = (size_t)(kUThreads / 32) * kRingRows * kDayRows * s.Fs * sizeof(float);
     int dev = 0, sms = 0, per_sm = 0;
-    TSVD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(kern, smem);
     TSVD_CUDA(cudaGetDevice(&dev));
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TSVD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kUThreads, smem));

@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(32 * kWideWarps) k_item_wide_pairs(DeviceState
 template <class Kern>
 unsigned wide_grid(Kern kern, uint32_t Fs, size_t smem) {
     int dev = 0, sms = 0, per_sm = 0;
-    TSVD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_dyn_smem(kern, smem);
     TSVD_CUDA(cudaGetDevice(&dev));
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TSVD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (int)(Fs / kWideV), smem));
