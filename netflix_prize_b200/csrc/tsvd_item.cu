@@ -70,6 +70,7 @@ enum {
     vSameT,     // the ratings of the same time bin
     vSameF,     // ... frequency bin
     vTarget,    // the raw rating (ordinal head)
+    vUnscale,   // the inverse of the pe row's scale
     vSlotOff,   // by slot (the round's bins, in order of their first rating): the row's offset,
     vSlotDec,   // ... a_f^(ratings of the bin) - 1
     vSlots,     // [0]: the number of slots
@@ -103,24 +104,6 @@ __host__ __device__ inline ItemSmem item_smem(uint32_t Fs, uint32_t NF, uint32_t
     L.pow = o;  o += 8 * 36;                        // a_i^n, a_f^n, a_i^n - 1, a_f^n - 1, n = 0 .. kRound; rounded a
     L.total = o;
     return L;
-}
-
-// d (16x8, FP32) += a (16x16, BF16, row-major) . b (16x8, BF16, column-major)
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// x = hi + lo + r in packed BF16 pairs (round to nearest even), |r| <= 2^-17 |x|.
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const float2 f = __bfloat1622float2(h);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
 // One producer's rows of a round, asked for a step ahead.
@@ -219,6 +202,10 @@ __device__ __forceinline__ void stage(const ItemCtx& c, uint32_t r, int pw, int 
             R.x[k].fma(h, R.c[k]);
         }
         R.x[k].store(pe + (uint32_t)j * P, lane);
+        float x[VPL];
+        R.x[k].to(x);
+        const float unscale = row_unscale(x);
+        if (lane == 0) V[vUnscale * kRound + j] = unscale;
     }
 }
 
@@ -234,16 +221,16 @@ __device__ __forceinline__ void make_m(const ItemCtx& c, uint32_t r, int pw, int
     {
         // Tiles of G = PE PE^T that hold every pair: rows 0-15 with columns 0-7,
         // 8-15, 16-23 (warps 0-2), rows 0-15 with 24-31, rows 16-31 with 16-23,
-        // 24-31 (warps 3-5). The products are of BF16 high and low parts (hi hi +
-        // hi lo + lo hi, error ~2^-16 of |pe_i||pe_j|), split on the way in: the
-        // warp-level MMAs, one per 40 cycles and scheduler, hide it. A lane reads 4
+        // 24-31 (warps 3-5), from FP16 parts, split on the way in. A lane reads 4
         // consecutive values as the k indices (2t, 2t+1, 2t+8, 2t+9) of a 16-column
         // step, for both operands alike, so a row's fragment serves as either.
         const int third = pw % 3;
         const bool low = pw >= 3;
         const int g = lane >> 2, t = lane & 3;
         const float* row = pe + (uint32_t)g * P + 4 * t;
-        float d[3][3][4] = {};
+        float d[3][3][4] = {}, scale[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) scale[x] = row_scale(V[vUnscale * kRound + g + 8 * x]);
 #pragma unroll 1
         for (int ks = third * (2 * VPL) / 3; ks < (third + 1) * (2 * VPL) / 3; ++ks) {
             // fragments of rows 0-7, 8-15, 16-23, 24-31: {lo pair, hi pair} of k
@@ -252,15 +239,15 @@ __device__ __forceinline__ void make_m(const ItemCtx& c, uint32_t r, int pw, int
             for (int x = 0; x < 4; ++x) {
                 if (x < 3 || low) {
                     const float4 v = *reinterpret_cast<const float4*>(row + (uint32_t)(8 * x) * P + 16 * ks);
-                    split_pair(v.x, v.y, h[x][0], l[x][0]);
-                    split_pair(v.z, v.w, h[x][1], l[x][1]);
+                    split_pair(v.x * scale[x], v.y * scale[x], h[x][0], l[x][0]);
+                    split_pair(v.z * scale[x], v.w * scale[x], h[x][1], l[x][1]);
                 }
             }
             const uint32_t ah[4] = {h[0][0], h[1][0], h[0][1], h[1][1]}, al[4] = {l[0][0], l[1][0], l[0][1], l[1][1]};
             auto tile = [&](float (&acc)[3][4], const uint32_t (&xh)[4], const uint32_t (&xl)[4], int b) {
-                mma_bf16(acc[0], xl, h[b][0], h[b][1]);
-                mma_bf16(acc[1], xh, l[b][0], l[b][1]);
-                mma_bf16(acc[2], xh, h[b][0], h[b][1]);
+                mma_f16(acc[0], xl, h[b][0], h[b][1]);
+                mma_f16(acc[1], xh, l[b][0], l[b][1]);
+                mma_f16(acc[2], xh, h[b][0], h[b][1]);
             };
             if (!low) {
                 tile(d[0], ah, al, 0);
@@ -291,13 +278,14 @@ __device__ __forceinline__ void make_m(const ItemCtx& c, uint32_t r, int pw, int
     const uint32_t bi = __float_as_uint(V[vBins * kRound + lane]);
     const unsigned after = ~((2u << lane) - 1u);
     const float* Gi = G + lane * kGPitch;
+    const float unscale = V[vUnscale * kRound + lane];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         const int j = pw + 6 * k;
         if (k < 5 || j < kRound) {
             const uint32_t bj = __float_as_uint(V[vBins * kRound + j]);
             const unsigned same = __float_as_uint(V[vSameF * kRound + j]);
-            const float g = (Gi[j] + Gi[kRound * kGPitch + j]) + Gi[2 * kRound * kGPitch + j];
+            const float g = ((Gi[j] + Gi[kRound * kGPitch + j]) + Gi[2 * kRound * kGPitch + j]) * unscale * V[vUnscale * kRound + j];
             const bool same_f = (same >> lane & 1u) != 0u, same_t = ((bi ^ bj) & 0xffu) == 0u;
             const float ai = c.apow[max(j - 1 - lane, 0)];
             const float af = c.fpow[__popc(same & after & ((1u << j) - 1u))];

@@ -1,5 +1,7 @@
 // The item stratum's light items (tsvd_item.cu, tsvd_item_tiles.cu).
 #pragma once
+#include <cuda_fp16.h>
+
 #include "tsvd_chain.cuh"
 
 namespace tsvd {
@@ -34,6 +36,44 @@ __device__ __forceinline__ float rounded_step(float d) {
     double r = x;
     for (int e = 0; e < 5; ++e) r = sqrt(r);
     return (float)(r - 1.0);
+}
+
+// ---------------------------------------------------------------------------
+// The dots pe_i . pe_k of a round by the warp-level MMAs, with the digits of FP32
+// products: a value is taken as the sum of two FP16 parts, 22 bits, and of the four
+// products all but the least. A row is scaled by a power of two first, its largest
+// value to 2^14 .. 2^15, so that a part's 2^-25 is at most 2^-39 of that value. (Two
+// BF16 parts hold 16 bits: the next rating's error was up to 2^-15 lr |pe_i||pe_k| of
+// the last one off. Three BF16 parts and six products took 99.5 ms for an epoch of
+// 100,480,507 ratings, f = 256, where two took 91.1.)
+// ---------------------------------------------------------------------------
+// A warp's row: the inverse of its scale. (Rows below 2^-112 are scaled as that.)
+template <int VPL>
+__device__ __forceinline__ float row_unscale(const float (&x)[VPL]) {
+    float m = fabsf(x[0]);
+#pragma unroll
+    for (int v = 1; v < VPL; ++v) m = fmaxf(m, fabsf(x[v]));
+    const uint32_t largest = __reduce_max_sync(kFull, __float_as_uint(m));
+    return __uint_as_float((max(largest >> 23, 15u) - 14u) << 23);
+}
+__device__ __forceinline__ float row_scale(float unscale) { return __uint_as_float(0x7f000000u - __float_as_uint(unscale)); }
+
+// Packed FP16 pairs of (x, y): the values rounded, and what that leaves rounded.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// d (16x8, FP32) += a (16x16, FP16, row-major) . b (16x8, FP16, column-major)
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // An item's biases, spread over a warp.

@@ -30,8 +30,8 @@ constexpr uint32_t kMS = kRound + 1;  // padded row stride of the round's system
 constexpr int kCW = 4;                // consumer warps
 constexpr int kPW = 8;                // producer warps
 constexpr int kItemThreads = (kCW + kPW) * 32;
-constexpr int kVecs = 9;              // per-rating vectors of a round
-// BF16 rows of the Gram operands: Fs values + 16 bytes, so that the eight
+constexpr int kVecs = 10;             // per-rating vectors of a round
+// FP16 rows of the Gram operands: Fs values + 16 bytes, so that the eight
 // 16-byte row segments an ldmatrix reads fall in distinct bank groups
 __host__ __device__ constexpr uint32_t hl_pitch(uint32_t Fs) { return Fs * 2 + 16; }
 static_assert(kPW * 4 == kRound, "each producer warp stages four of the round's ratings");
@@ -46,7 +46,7 @@ __host__ __device__ inline ItemSmem item_smem(uint32_t Fs, uint32_t NF) {
     L.qfs = o;  o += NF * (Fs + 4);             // the item's q^f rows, padded
     L.qsh = o;  o += Fs;                        // q at the round's start
     L.buf = o;  o += 2 * kRound * (Fs + 4);     // two rounds of pe rows + {bu_t, cu_t, res, key}
-    L.hl = o;   o += 2 * kRound * (Fs / 2 + 4); // BF16 high and low parts of the produced round's pe rows
+    L.hl = o;   o += 2 * kRound * (Fs / 2 + 4); // FP16 high and low parts of the produced round's pe rows
     L.mbuf = o; o += 2 * kRound * kMS;          // two rounds of the system M (row j: M_j,i)
     L.vec = o;  o += 2 * kVecs * kRound;        // two rounds of per-rating weights
     L.pd = o;   o += kCW * 2 * kRound;          // consumers' partial dots
@@ -169,42 +169,37 @@ __device__ void item_light(const DeviceState& s, const EpochParams& p, const Bf1
     store_item_state(s, i, lane, st);
 }
 
-// x = hi + lo + r with hi, lo in BF16 (round to nearest even), |r| <= 2^-17 |x|.
-__device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bfloat16& lo) {
-    hi = __float2bfloat16_rn(x);
-    lo = __float2bfloat16_rn(x - __bfloat162float(hi));
-}
-
-// One staged rating: its FP32 pe row (for the consumers) and the BF16 high and
-// low parts of it (the Gram operands), each element split once.
+// One staged rating: its FP32 pe row (for the consumers) and the FP16 high and
+// low parts of it, scaled (the Gram operands), each element split once. Returns the
+// inverse of the scale.
 template <int VPL>
-__device__ __forceinline__ void stage_row(float* row, uint8_t* hi_row, uint8_t* lo_row, int lane,
-                                          const float (&pe)[VPL]) {
+__device__ __forceinline__ float stage_row(float* row, uint8_t* hi_row, uint8_t* lo_row, int lane,
+                                           const float (&pe)[VPL]) {
+    const float unscale = row_unscale(pe), sc = row_scale(unscale);
     if constexpr (VPL % 4 == 0) {
 #pragma unroll
         for (int c = 0; c < VPL / 4; ++c) {
             const int col = c * 128 + lane * 4;
             const float4 x = make_float4(pe[4 * c], pe[4 * c + 1], pe[4 * c + 2], pe[4 * c + 3]);
             *reinterpret_cast<float4*>(row + col) = x;
-            __nv_bfloat16 h[4], l[4];
-            split_bf16(x.x, h[0], l[0]);
-            split_bf16(x.y, h[1], l[1]);
-            split_bf16(x.z, h[2], l[2]);
-            split_bf16(x.w, h[3], l[3]);
-            *reinterpret_cast<uint2*>(hi_row + 2 * col) = *reinterpret_cast<const uint2*>(h);
-            *reinterpret_cast<uint2*>(lo_row + 2 * col) = *reinterpret_cast<const uint2*>(l);
+            uint2 h, l;
+            split_pair(x.x * sc, x.y * sc, h.x, l.x);
+            split_pair(x.z * sc, x.w * sc, h.y, l.y);
+            *reinterpret_cast<uint2*>(hi_row + 2 * col) = h;
+            *reinterpret_cast<uint2*>(lo_row + 2 * col) = l;
         }
     } else {
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
             const int col = Row<VPL>::elem(lane, v);
             row[col] = pe[v];
-            __nv_bfloat16 h, l;
-            split_bf16(pe[v], h, l);
-            reinterpret_cast<__nv_bfloat16*>(hi_row)[col] = h;
-            reinterpret_cast<__nv_bfloat16*>(lo_row)[col] = l;
+            const float x = pe[v] * sc;
+            const __half h = __float2half_rn(x);
+            reinterpret_cast<__half*>(hi_row)[col] = h;
+            reinterpret_cast<__half*>(lo_row)[col] = __float2half_rn(x - __half2float(h));
         }
     }
+    return unscale;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -213,15 +208,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
-}
-
-// d (16x8, FP32) += a (16x16, BF16, row-major) . b (16x8, BF16, column-major)
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-        "{%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
 template <int VPL, bool BF>
@@ -370,15 +356,20 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
                     px0[v] = px0[v] + d0 * py0[v];
                     px1[v] = px1[v] + d1 * py1[v];
                 }
-                stage_row<VPL>(dst + (size_t)j0 * stride, hl + (size_t)j0 * hp, hl + (size_t)(kRound + j0) * hp, lane, px0);
-                stage_row<VPL>(dst + (size_t)j1 * stride, hl + (size_t)j1 * hp, hl + (size_t)(kRound + j1) * hp, lane, px1);
+                const float s0 = stage_row<VPL>(dst + (size_t)j0 * stride, hl + (size_t)j0 * hp,
+                                                 hl + (size_t)(kRound + j0) * hp, lane, px0);
+                const float s1 = stage_row<VPL>(dst + (size_t)j1 * stride, hl + (size_t)j1 * hp,
+                                                 hl + (size_t)(kRound + j1) * hp, lane, px1);
 #pragma unroll
                 for (int v = 0; v < VPL; ++v) {
                     x2[v] = x2[v] + d2 * y2[v];
                     x3[v] = x3[v] + d3 * y3[v];
                 }
-                stage_row<VPL>(dst + (size_t)j2 * stride, hl + (size_t)j2 * hp, hl + (size_t)(kRound + j2) * hp, lane, x2);
-                stage_row<VPL>(dst + (size_t)j3 * stride, hl + (size_t)j3 * hp, hl + (size_t)(kRound + j3) * hp, lane, x3);
+                const float s2 = stage_row<VPL>(dst + (size_t)j2 * stride, hl + (size_t)j2 * hp,
+                                                 hl + (size_t)(kRound + j2) * hp, lane, x2);
+                const float s3 = stage_row<VPL>(dst + (size_t)j3 * stride, hl + (size_t)j3 * hp,
+                                                 hl + (size_t)(kRound + j3) * hp, lane, x3);
+                if (lane < 4) V[9 * kRound + pw + kPW * lane] = lane == 0 ? s0 : lane == 1 ? s1 : lane == 2 ? s2 : s3;
             }
             // all rows of the round are in place before the Gram products
             asm volatile("bar.sync 2, %0;" ::"r"(kPW * 32) : "memory");
@@ -386,8 +377,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
             // the round's ratings of each frequency bin (valid ratings only)
             const unsigned same = __match_any_sync(kFull, valid ? fbl : 64u + (uint32_t)lane);
             if (pw < 6) {
-                // G = PE PE^T on the tensor cores, from BF16 high and low
-                // parts of pe (three products: error ~2^-16 of |pe_i||pe_j|).
+                // G = PE PE^T on the tensor cores, from FP16 high and low parts.
                 // Tile pw of the six 16x8 tiles (rows x columns) that hold
                 // every pair row < column.
                 const int mt = pw < 4 ? 0 : 1, nt = pw < 4 ? pw : pw - 2;
@@ -411,10 +401,9 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
                         ldmatrix_x4(ah, a_hi + kb);
                         ldmatrix_x4(al, a_lo + kb);
                         ldmatrix_x4(bb, b_hl + kb);
-                        const uint32_t bh[2] = {bb[0], bb[1]}, bl[2] = {bb[2], bb[3]};
-                        mma_bf16(d[3 * hh], al, bh);
-                        mma_bf16(d[3 * hh + 1], ah, bl);
-                        mma_bf16(d[3 * hh + 2], ah, bh);
+                        mma_f16(d[3 * hh], al, bb[0], bb[1]);
+                        mma_f16(d[3 * hh + 1], ah, bb[2], bb[3]);
+                        mma_f16(d[3 * hh + 2], ah, bb[0], bb[1]);
                     }
                 }
                 // The round's errors solve err = C - M err with M unit lower
@@ -424,13 +413,14 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
                 // This lane's four entries (i, j) give M_ji and M_ij = 0.
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float g = ((d[0][e] + d[1][e]) + (d[3][e] + d[4][e])) + (d[2][e] + d[5][e]);
                     const int ii = mt * 16 + gid + 8 * (e >> 1), jj = nt * 8 + 2 * tig + (e & 1);
                     const uint32_t ki = __shfl_sync(kFull, mine.key, ii), kj = __shfl_sync(kFull, mine.key, jj);
                     const unsigned samej = __shfl_sync(kFull, same, jj);
                     if (ii < jj) {
                         float v = 0.0f;
                         if (jj < (int)m) {
+                            const float g = (((d[0][e] + d[1][e]) + (d[3][e] + d[4][e])) + (d[2][e] + d[5][e])) *
+                                            V[9 * kRound + ii] * V[9 * kRound + jj];
                             const float cui = dst[(size_t)ii * stride + Fs + 1], cuj = dst[(size_t)jj * stride + Fs + 1];
                             const bool same_f = rec_fbin(ki) == rec_fbin(kj), same_t = rec_tbin(ki) == rec_tbin(kj);
                             const float bias_lr = p.lr_ib + (same_t ? p.lr_ti : 0.0f) + (same_f ? p.lr_ibf : 0.0f);

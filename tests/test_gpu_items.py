@@ -124,3 +124,77 @@ def test_thresholds_that_take_the_same_items_give_the_same_bits(f):
         for g in got[1:]:
             for n in ITEM_PARAMS:
                 assert np.array_equal(g[n], got[0][n]), (same, n)
+
+
+ROUND_COUNTS = [64, 32, 20, 2]
+
+
+def one_bin_rounds():
+    """Item k is rated by the first ROUND_COUNTS[k] of 64 users, each rating in a time
+    bin of its own (of 64) and in frequency bin 0."""
+    u = np.concatenate([np.arange(c) for c in ROUND_COUNTS])
+    i = np.repeat(np.arange(len(ROUND_COUNTS)), ROUND_COUNTS)
+    o = np.lexsort((i, u))
+    u, i = u[o], i[o]
+    n = len(ROUND_COUNTS) + 1
+    tr = Dataset.from_ratings(u, i, 1 + (u * 7 + i * 3) % 5, 20 * u + i, 64, n, "rounds")
+    pr = Dataset.from_ratings(np.arange(64), np.full(64, n - 1), np.full(64, 3), 20 * np.arange(64) + 19, 64, n, "rounds_pr")
+    return tr, pr
+
+
+def chain_errors(p, q, h, y, lr, g, th):
+    """The errors of an item's ratings, one after another in 64 bits."""
+    out = []
+    for x, t in zip(p, y):
+        e = g + x @ (q + h) - t
+        if th is not None:
+            c = np.concatenate([[0.0], 1 / (1 + np.exp(-(th - (e + t)))), [1.0]])
+            e = 1.0 - c[t] - c[t - 1]
+        q, h = q - lr * e * x, h - lr * e * x
+        out.append(e)
+    return np.array(out)
+
+
+@pytest.mark.parametrize("f,low_memory,ordinal", [(32, True, False), (64, True, False), (96, True, False), (128, True, False),
+                                                  (160, True, False), (224, True, False), (256, True, False),
+                                                  (20, False, False), (160, False, False), (256, False, False),
+                                                  (20, True, True), (128, True, True), (200, True, True)])
+def test_a_round_keeps_the_digits_of_its_rows(f, low_memory, ordinal):
+    """Rows of equal values and steps of the size of 1 / |row|^2, where what a product of
+    two rows loses is lost in every column alike and moves the next rating's error by
+    as much. The errors are read from the time-bin biases, one a rating (lr_ti = 1).
+
+    Tolerance: a score of up to 4 comes from some 20 roundings (a lane's share of the
+    columns, five or six levels of sums, the biases, the system's row), half an ulp,
+    2.4e-7, each: 4.8e-6. The head's gradient has half that slope at most, but is a
+    quotient by a probability above 0.05 of three roundings of 6e-8: 2.4e-6 + 3.6e-6.
+    Products of two 8-bit parts of each value are 1.8e-5 (with the head) and 7e-5 off."""
+    tr, pr = one_bin_rounds()
+    names = ("lr_u", "lr_u2", "lr_ud", "lr_ub", "lr_ubd", "lr_y", "lr_yb", "lr_yd", "lr_ta", "lr_tu", "lr_cu", "lr_ib", "lr_ibf",
+             "reg_i", "reg_iqf")
+    value = np.float32(1.003898)  # 2^-8 and 2^-17 past a number of 8 bits
+    lr = float(np.float32((1.2 if ordinal else 0.45) / (f * float(value) ** 2)))
+    th = (0.5, 1.25, 3.75, 5.5)
+    cfg = run_lm(f, 1, n_time_bins=64, low_memory=low_memory).replace(
+        lr_i=lr, lr_iqf=lr, lr_ti=1.0, ordinal_head=OrdinalHeadConfig(th, 0.001, 0.0, 0.0) if ordinal else None,
+        **{n: 0.0 for n in names})
+    n, nf = tr.n_items, cfg.n_freq_bins
+    rng = np.random.default_rng(6)
+    init = {"ufeat": np.full((64, f), value, np.float32), "ufeat2": np.zeros((64, f), np.float32),
+            "ifeat": rng.normal(0, 0.01, (n, f)).astype(np.float32), "yfeat": np.zeros((n, f), np.float32),
+            "ifeat_freq": rng.normal(0, 0.01, (n * nf, f)).astype(np.float32)}
+    if not low_memory:
+        init["yfeat_day"] = np.zeros((n, f), np.float32)
+    for heavy in (1, 100000):
+        m = TxModel(tr, MaskedDataset(pr), cfg, heavy_item_ratings=heavy)
+        for k, v in init.items():
+            m.set_param(k, v)
+        m.fit_epoch(tr, pr, 1)
+        assert np.array_equal(m.get_param("ufeat"), init["ufeat"])
+        g = float(np.asarray(m.get_param("gbias")).ravel()[0])
+        got = -np.asarray(m.get_param("bit_bin"), np.float64).reshape(n, 64)
+        for k, c in enumerate(ROUND_COUNTS):
+            y = 1 + (np.arange(c) * 7 + k * 3) % 5
+            want = chain_errors(init["ufeat"][:c].astype(np.float64), init["ifeat"][k].astype(np.float64),
+                                init["ifeat_freq"][k * nf].astype(np.float64), y, lr, g, np.array(th) if ordinal else None)
+            assert np.max(np.abs(got[k, :c] - want)) < (6e-6 if ordinal else 4.8e-6), (heavy, c)
