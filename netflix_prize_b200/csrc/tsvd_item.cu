@@ -594,6 +594,7 @@ __global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_roun
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t Fs = s.Fs, NF = s.NF, T = s.T;
     ItemCtx c{s, p, bf, smem, item_smem(Fs, NF, CW), 0, 0, 0, row_pitch(Fs), nullptr, nullptr, nullptr, nullptr, s.raw != nullptr};
+    if (threadIdx.x == 64) sh_next[1] = atomicAdd(&s.counters[2], 1u);
     if (threadIdx.x < 2) decay_powers<kRound>(smem + c.L.pow + threadIdx.x * 144, p, threadIdx.x == 1);
     // the zero columns of an odd width (those of q and q^f come with each item: an
     // update by a weight that is not finite leaves them not zero)
@@ -606,8 +607,11 @@ __global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_roun
     __syncthreads();
     const int pw = warp - CW;
     float* bias = smem + c.L.bias;
-    // the first items one per CTA (heaviest first), then from the counter
-    uint32_t k = blockIdx.x;
+    // Items heaviest first, each to the next block that is free. Where several passes
+    // share the GPU (tsvd_group.cu) not every block of a pass is there from the start,
+    // and one that owned an item would keep it waiting (eight variants of 1 M ratings,
+    // up to 128 columns: 6.9 ms an epoch with the first items bound to blocks, 6.4 so).
+    uint32_t k = sh_next[1];
     // light items one warp each; with the per-day rows every item goes in rounds
     const uint32_t heavy_min = MODE == kPerDay ? 1u : max(s.heavy_min, 1u);
     for (uint32_t turn = 0; k < s.n_item_work; ++turn) {
@@ -675,7 +679,7 @@ __global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_roun
             if (pw == 7) make_vectors(c, 0, lane, rec);
             if (pw == 6) {
                 if (lane == 0) {
-                    sh_next[turn & 1] = gridDim.x + atomicAdd(&s.counters[2], 1u);
+                    sh_next[turn & 1] = atomicAdd(&s.counters[2], 1u);
                     bias[0] = __ldcg(s.ibias + i);
                 }
                 for (uint32_t e = lane; e < 64; e += 32) {
@@ -739,7 +743,7 @@ __global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_roun
     }
     if constexpr (MODE != kPerDay) {
         if (warp > 0) {
-            if (lane == 0) k = gridDim.x + atomicAdd(&s.counters[2], 1u);
+            if (lane == 0) k = atomicAdd(&s.counters[2], 1u);
             k = __shfl_sync(kFull, k, 0);
         }
         light_items<VPL, MODE == kBf16>(s, p, bf, k, lane, smem + warp * kLightRows * 2 * Fs);

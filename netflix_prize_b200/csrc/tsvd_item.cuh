@@ -284,7 +284,7 @@ __device__ __forceinline__ void light_items(const DeviceState& s, const EpochPar
         const uint32_t i = s.item_work[k];
         if (s.item_off[i] == s.item_off[i + 1]) break;  // no ratings, and none after it
         item_pairs<VPL, BF>(s, p, bf, i, lane, ring);
-        if (lane == 0) k = gridDim.x + atomicAdd(&s.counters[2], 1u);
+        if (lane == 0) k = atomicAdd(&s.counters[2], 1u);
         k = __shfl_sync(kFull, k, 0);
     }
 }
