@@ -3,9 +3,12 @@ import numpy as np
 import pytest
 import torch
 
+from netflix_prize_b200.abi import PREC_BF16_READ_ALL
 from netflix_prize_b200.config import OrdinalHeadConfig, run_lm
 from netflix_prize_b200.data import Dataset, MaskedDataset
 from netflix_prize_b200.model import TxModel
+from oracle import pyoracle as po
+from tests.test_gpu_chains import ITEM_COUNTS, counted_items
 
 pytestmark = pytest.mark.gpu
 
@@ -198,3 +201,78 @@ def test_a_round_keeps_the_digits_of_its_rows(f, low_memory, ordinal):
             want = chain_errors(init["ufeat"][:c].astype(np.float64), init["ifeat"][k].astype(np.float64),
                                 init["ifeat_freq"][k * nf].astype(np.float64), y, lr, g, np.array(th) if ordinal else None)
             assert np.max(np.abs(got[k, :c] - want)) < (6e-6 if ordinal else 4.8e-6), (heavy, c)
+
+
+FROZEN = {n: 0.0 for n in ("lr_u", "lr_u2", "lr_ub", "lr_ubd", "lr_y", "lr_yb", "lr_ta", "lr_tu", "lr_cu")}
+# strong updates and decays of rows and bins, as in the tests of the item stratum without the head
+STRONG = dict(lr_ti=0.002, lr_ibf=0.003, lr_iqf=0.004, reg_iqf=0.05, reg_i=0.05, sigma_u=0.1, sigma_i=0.1, sigma_iqf=0.1)
+
+
+@pytest.mark.parametrize("heavy", [1, 40, 100000])
+@pytest.mark.parametrize("f", [20, 64, 96, 160, 256])
+def test_item_stratum_with_the_ordinal_head(f, heavy):
+    """Items in rounds and by pairs against their chains in 64 bits (src/tsvdx4p.rs:644-762
+    with the head's gradient, src/lib.rs:562-598), users frozen; the bound of one epoch's
+    parity, 2e-5."""
+    tr, pr = counted_items(ITEM_COUNTS, 200, 5)
+    th = np.array([0.5, 1.25, 3.75, 5.5])
+    cfg = run_lm(f, 1, n_time_bins=48).replace(ordinal_head=OrdinalHeadConfig(tuple(th), 0.001, 0.0, 0.0), **STRONG, **FROZEN)
+    m = TxModel(tr, MaskedDataset(pr), cfg, heavy_item_ratings=heavy)
+    rng = np.random.default_rng(8)
+    m.set_param("ufeat2", rng.normal(0, 0.05, (200, f)).astype(np.float32))
+    names = ["ufeat", "ufeat2", "tu_mean"] + ITEM_PARAMS
+    P = {n: np.asarray(m.get_param(n), np.float64) for n in names}
+    m.fit_epoch(tr, pr, 1)
+    yc, ycb = np.asarray(m.get_param("ycache"), np.float64), np.asarray(m.get_param("ycache_bias"), np.float64)
+    g = float(np.asarray(m.get_param("gbias")).ravel()[0])
+    n, nf, T = tr.n_items, cfg.n_freq_bins, cfg.n_time_bins
+    qf, bt, bf = P["ifeat_freq"].reshape(n, nf, f), P["bit_bin"].reshape(n, T), P["ibias_freq"].reshape(n, nf)
+    q, ib = P["ifeat"].reshape(n, f), P["ibias"].ravel()
+    _, at, day_cnt = np.unique(np.concatenate([tr.user_idxs, pr.user_idxs]) * 10000
+                               + np.concatenate([tr.dates, pr.dates]).astype(np.int64), return_inverse=True, return_counts=True)
+    fbin = np.minimum(np.log2(day_cnt[at[:len(tr.user_idxs)]]).astype(int), nf - 1)
+    assert len(np.unique(fbin)) > 2
+    day_range = int(max(tr.dates.max(), pr.dates.max())) + 1
+    for i in range(n):
+        rows = np.nonzero(tr.item_idxs == i)[0]
+        for t in rows[np.argsort(tr.user_idxs[rows], kind="stable")]:
+            u, day, b = tr.user_idxs[t], int(tr.dates[t]), fbin[t]
+            tb = min(day * T // day_range, T - 1)
+            dt = day - P["tu_mean"][u]
+            dv = np.sign(dt) * abs(dt) ** np.float64(np.float32(cfg.beta))
+            pe = P["ufeat"][u] + yc[u] + dv * P["ufeat2"][u]
+            x = g + ycb[u] + ib[i] + bt[i, tb] + bf[i, b] + pe @ (q[i] + qf[i, b])
+            c = np.concatenate([[0.0], 1 / (1 + np.exp(-(th - x))), [1.0]])
+            y = int(tr.raw_ratings[t])
+            e = (c[y] * (1 - c[y]) - c[y - 1] * (1 - c[y - 1])) / max(c[y] - c[y - 1], 1e-6)
+            ib[i] -= cfg.lr_ib * e
+            bt[i, tb] -= cfg.lr_ti * e
+            bf[i, b] -= cfg.lr_ibf * e
+            q[i], qf[i, b] = (q[i] - cfg.lr_i * (e * pe + cfg.reg_i * q[i]),
+                              qf[i, b] - cfg.lr_iqf * (e * pe + cfg.reg_iqf * qf[i, b]))
+    for name, want in (("ifeat", q), ("ifeat_freq", qf), ("ibias", ib), ("bit_bin", bt), ("ibias_freq", bf)):
+        assert np.max(np.abs(np.asarray(m.get_param(name), np.float64).ravel() - want.ravel())) < 2e-5, name
+
+
+@pytest.mark.parametrize("heavy", [1, 40, 100000])
+@pytest.mark.parametrize("f", [20, 64, 128, 160, 256])
+def test_item_stratum_with_rounded_user_rows(f, heavy):
+    """User rows that are BF16 numbers already: the precision form that reads them as
+    such is, users frozen, within the bound of FP32 parity of the oracle's epoch."""
+    tr, pr = counted_items(ITEM_COUNTS, 200, 5)
+    cfg = run_lm(f, 1, n_time_bins=48).replace(**STRONG, **FROZEN)
+    rng = np.random.default_rng(9)
+    init = {n: torch.as_tensor(rng.normal(0, sd, (200, f)), dtype=torch.bfloat16).float().numpy()
+            for n, sd in (("ufeat", 0.1), ("ufeat2", 0.05))}
+    init["yfeat"] = np.zeros((tr.n_items, f), np.float32)
+    o = po.OracleModel(tr, MaskedDataset(pr), cfg)
+    m = TxModel(tr, MaskedDataset(pr), cfg, precision=PREC_BF16_READ_ALL, heavy_item_ratings=heavy)
+    for n, v in init.items():
+        o.set_param(n, v)
+        m.set_param(n, v)
+    o.fit_epoch(1, po.SCHED_P, nsvd_norm_exp=1.0, n_threads=1)
+    m.fit_epoch(tr, pr, 1)
+    assert np.array_equal(m.get_param("ufeat"), init["ufeat"])
+    for n in ITEM_PARAMS:
+        a, b = np.asarray(m.get_param(n), np.float64).ravel(), np.asarray(o.get_param(n), np.float64).ravel()
+        assert np.max(np.abs(a - b) - 1e-5 * np.abs(b)) < 2e-5, n
