@@ -55,8 +55,6 @@ __host__ __device__ constexpr int group_warps(int vpl) { return (vpl + lane_cols
 __host__ __device__ constexpr int groups(int vpl) { return vpl >= 5 ? 1 : 2; }
 __host__ __device__ constexpr int consumers(int vpl) { return groups(vpl) * group_warps(vpl); }
 __host__ __device__ constexpr int item_threads(int vpl) { return (consumers(vpl) + kPW) * 32; }
-// CTAs per SM that the registers are bounded for
-__host__ __device__ constexpr int item_ctas(int vpl) { return 1; }
 
 // A round's vectors, by rating unless said otherwise.
 enum {
@@ -586,7 +584,7 @@ __device__ __forceinline__ void consume(const ItemCtx& c, uint32_t r, int cw, in
 }
 
 template <int VPL, int MODE>
-__global__ void __launch_bounds__(item_threads(VPL), item_ctas(VPL)) k_item_rounds(DeviceState s, EpochParams p,
+__global__ void __launch_bounds__(item_threads(VPL), 1) k_item_rounds(DeviceState s, EpochParams p,
                                                                                    Bf16Copies bf) {
     extern __shared__ __align__(16) float smem[];
     __shared__ uint32_t sh_next[2];
@@ -756,10 +754,9 @@ void launch_item(tsvd_model* m, const DeviceState& s, const EpochParams& p, cons
     const size_t smem = std::max<size_t>(item_smem(s.Fs, s.NF, consumers(VPL)).total,
                                          light_smem(item_threads(VPL) / 32, s.Fs)) * sizeof(float);
     allow_dyn_smem(kern, smem);
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, sms = 0;
     TSVD_CUDA(cudaGetDevice(&dev));
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    TSVD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, item_threads(VPL), smem));
     kern<<<(unsigned)sms, item_threads(VPL), smem, m->stream>>>(s, p, bf);
     TSVD_CUDA(cudaGetLastError());
     m->launches++;

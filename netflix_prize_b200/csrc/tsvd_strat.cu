@@ -40,7 +40,6 @@ __global__ void k_to_bf16(const float* __restrict__ src, uint64_t rows, uint32_t
     }
 }
 
-// The item rows a user-stratum rating reads: q_i and q^f_i of frequency bin fb.
 // qe0 = q_i + q^f_{i,0}: with low_memory the user stratum trains frequency bin
 // 0 only (src/tsvdx4p.rs:504-531) and reads the two rows only as this sum.
 // In the precision form both addends are rounded to BF16 first.
@@ -55,13 +54,6 @@ __global__ void k_make_qe0(const float* __restrict__ ifeat, const float* __restr
 }
 
 void make_qe0(tsvd_model* m, bool bf16);
-
-
-// err of a rating: score - residual, or with the ordinal head the gradient of
-// -log P(y) in the score (src/tx.rs:963-972); `target` is then the raw rating.
-__device__ __forceinline__ float rating_err(const DeviceState& s, const float (&th)[4], float score, float target) {
-    return s.raw ? ordinal_grad(th, score, (int)target) : score - target;
-}
 
 // ---------------------------------------------------------------------------
 // NSVD1 delta sums per item in two fixed-order levels: fixed chunks of
@@ -351,8 +343,6 @@ __global__ void __launch_bounds__(kThreads) k_user_strat_wide(DeviceState s, Epo
     using R8 = Row<kWV>;
     const int lane = threadIdx.x & 31;
     const uint32_t Fs = s.Fs, T = s.T, NF = s.NF;
-    float th[4];
-    load_thresholds(s, th);
     for (;;) {
         uint32_t k = 0;
         if (lane == 0) k = atomicAdd(&s.counters[0], 1u);
@@ -433,7 +423,7 @@ __global__ void __launch_bounds__(kThreads) k_user_strat_wide(DeviceState s, Epo
                     for (int v = 0; v < kWV; ++v) part += qe[v] * ((pu[v] + su[v]) + dv * p2[v]);
                 }
                 const float dot = warp_sum(part);
-                const float err = rating_err(s, th, gb + bu_t + bi_t * cu_t + dot, r.res);
+                const float err = gb + bu_t + bi_t * cu_t + dot - r.res;
                 ub -= p.lr_ub * err;
                 {
                     const float nb = but - p.lr_tu * err;
@@ -490,8 +480,6 @@ __global__ void __launch_bounds__(kThreads) k_item_wide(DeviceState s, EpochPara
     using R8 = Row<kWV>;
     const int lane = threadIdx.x & 31;
     const uint32_t Fs = s.Fs, NF = s.NF;
-    float th[4];
-    load_thresholds(s, th);
     const float gb = s.gbias;
     for (;;) {
         uint32_t k = 0;
@@ -533,7 +521,7 @@ __global__ void __launch_bounds__(kThreads) k_item_wide(DeviceState s, EpochPara
                     for (int v = 0; v < kWV; ++v) part += (x[v] + r.dev * y[v]) * (q[v] + qf[v]);
                 }
                 const float dot = warp_sum(part);
-                const float err = rating_err(s, th, gb + bu_t + bi_t * cu_t + dot, r.res);
+                const float err = gb + bu_t + bi_t * cu_t + dot - r.res;
                 const float ec = err * cu_t;
                 st.ib -= p.lr_ib * ec;
                 const float nb = bit - p.lr_ti * ec;
@@ -686,7 +674,6 @@ __global__ void k_reset_users(DeviceState s, const uint32_t* __restrict__ users,
 
 // (With the per-day terms the fold-in's yfeat_day deltas land in dyd_fix,
 // which the next stratified epoch clears before its user stratum.)
-template <int VPL>
 void foldin_launch(tsvd_model* m, const EpochParams& p, const uint32_t* d_users, uint32_t n) {
     if (m->d.dyd_fix) {
         launch_user_days(m, m->d, p, d_users, n);
@@ -726,7 +713,6 @@ void shard_user_launch(tsvd_model* m, const EpochParams& p, const uint32_t* work
     m->launches++;
 }
 
-template <int VPL, bool DAY>
 void shard_item_launch(tsvd_model* m, const EpochParams& p, const uint32_t* work, uint32_t n) {
     DeviceState s = m->d;
     s.item_work = work;
@@ -812,10 +798,9 @@ extern "C" int tsvd_foldin(tsvd_model* m, const uint32_t* users, uint64_t n, uin
         }
         EpochParams p = make_params(m);
         p.use_ycache = m->cfg.full_su ? 1 : 0;
-        const int vpl = (int)(m->d.Fs / 32);
         for (uint32_t k = 0; k < passes; ++k) {
             TSVD_CUDA(cudaMemsetAsync(m->d.counters, 0, 64, m->stream));
-            TSVD_DISPATCH(vpl, (foldin_launch<V>(m, p, du.as<uint32_t>(), (uint32_t)n)));
+            foldin_launch(m, p, du.as<uint32_t>(), (uint32_t)n);
         }
         TSVD_CUDA(cudaStreamSynchronize(m->stream));
     });
@@ -928,12 +913,7 @@ extern "C" int tsvd_shard_item_block(tsvd_model* m, uint32_t i_lo, uint32_t i_hi
             block_work(i_lo, i_hi, [&](uint32_t i) { return m->h_item_off[i + 1] - m->h_item_off[i]; });
         upload_work(m, w);
         const EpochParams p = make_params(m);
-        const int vpl = (int)std::min<uint32_t>(s.Fs / 32, 8);
-        if (s.dyd_fix) {
-            TSVD_DISPATCH(vpl, (shard_item_launch<V, true>(m, p, m->m_shard_work.as<uint32_t>(), (uint32_t)w.size())));
-        } else {
-            TSVD_DISPATCH(vpl, (shard_item_launch<V, false>(m, p, m->m_shard_work.as<uint32_t>(), (uint32_t)w.size())));
-        }
+        shard_item_launch(m, p, m->m_shard_work.as<uint32_t>(), (uint32_t)w.size());
         TSVD_CUDA(cudaStreamSynchronize(m->stream));
         finish_epoch(m);
     });
