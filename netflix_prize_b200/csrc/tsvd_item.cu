@@ -40,6 +40,10 @@ constexpr int kRound = 32;  // ratings per round
 // Rows from this many 32-column stripes on go to tsvd_item_tiles.cu where it
 // takes them: its round is bound by shared-memory traffic that this kernel has
 // more of (f = 256, hottest item of 476,450 ratings: 127 against 150 ns a rating).
+// Item pass there and here, ms, of 25 M ratings (of 1 M): 256 columns 15.8 and 19.8
+// (1.27, 1.50), 224 16.4 and 16.8 (1.28, 1.29), 192 15.4 and 14.0 (1.21, 1.07), 160
+// 14.3 and 13.5 (1.14, 1.03): the line is drawn by the widest rows, and 160 and 192
+// columns are on its slower side.
 constexpr int kTilesFrom = 5;
 constexpr int kPW = 8;      // producer warps
 constexpr int kGPitch = kRound + 2;  // row stride of the pairs' dots

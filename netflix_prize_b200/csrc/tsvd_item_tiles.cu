@@ -562,9 +562,8 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
                 // earlier rating of the chunk updated takes that value from
                 // registers, and the chunk's rows are stored at its end.
                 if (warp >= 2) {
-                    // item biases, beside the q and q^f updates of warps 0
-                    // and 1 (at f <= 64 warps 2 and 3 hold no stripes): warp 2
-                    // the item bias and the time-bin biases, warp 3 the
+                    // item biases, beside the warps' own stripes: warp 2 the
+                    // item bias and the time-bin biases, warp 3 the
                     // frequency-bin biases
                     if (warp == 2) {
                         const float sw = warp_sum(sv[2 * kRound + lane]);

@@ -193,8 +193,11 @@ uint32_t rounded_decay_min_for(const tsvd_model* m) {
 // GPU less, but its chain is longer. The line is where a light item's chain is
 // about as long as the pass, in shares of the ratings an SM gets: rows up to 128
 // columns (25 M ratings, f = 64) 9.9 ms at a quarter (42,000), 11.5 at 20,000,
-// 13.0 at 60,000; wider rows (f = 256) 16.9 ms at a twentieth (8,000), 19.9 at
-// 20,000, and 60.4 at 32,768 of 100 M.
+// 13.0 at 60,000. Wider rows: a twentieth (8,446 of 25 M) 15.8 ms at 256 columns,
+// 16.4 at 224, 15.4 at 192 and 14.3 at 160; 4,000 takes 0.1 to 0.3 ms more, 16,000
+// 0.2 less to none, 32,768 2.7 to 3.7 more (60.4 ms at 32,768 of 100 M). With the
+// ordinal head, whose rounds are another kernel's, the twentieth is low (200 columns:
+// 59.3 ms, 52.2 at 42,000).
 uint32_t heavy_min_for(const tsvd_model* m) {
     int sms = 0;
     TSVD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device));

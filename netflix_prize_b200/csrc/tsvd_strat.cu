@@ -10,10 +10,10 @@
 // No two work units touch the same parameter and every sum has a fixed
 // order, so a run is bitwise reproducible.
 //
-// Precision form: with BF16 read copies, the frozen tables a stratum only
-// reads are gathered as BF16 (item rows q_i, q^f_{i,0} and y_j; optionally
-// the user rows p_u, p2_u, ycache_u of the item stratum) and widened to FP32
-// for accumulation; masters stay FP32 and are the only tables written.
+// Precision form: the frozen tables a stratum only reads are rounded to BF16
+// (y_j, gathered as BF16; q_i and q^f_{i,0}, whose sum is read as FP32;
+// optionally p_u + ycache_u and p2_u in the item stratum, gathered as BF16)
+// and accumulated in FP32; masters stay FP32 and are the only tables written.
 #include <algorithm>
 #include <functional>
 #include <mutex>

@@ -11,10 +11,8 @@
 // the day's bias and c_u. One reduction of three sums (two dots and qe_0 . qe_1)
 // replaces two dependent ones, and the rows are read and scaled once per pair.
 //
-// Larger blocks cost no fewer instructions per rating and lose more than they
-// save: a loop of about 180 instructions stays in the instruction cache next to
-// the schedulers, one of 500 (blocks of four) waited 3.5 cycles for every
-// instruction it issued.
+// Larger blocks cost no fewer instructions per rating and a longer loop: blocks of
+// four took 26.8 ms at 100,480,507 ratings, f = 256, where pairs take 16.0.
 //
 // The rows come through a ring of shared-memory slots per warp, asked for
 // kAheadRows ratings ahead, so their latency takes no registers.
