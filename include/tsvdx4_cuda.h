@@ -153,7 +153,7 @@ typedef struct tsvd_gpu_options {
                                 32 ratings solved together), the others one
                                 warp each; 0 (or INT32_MAX) = default: a share
                                 of the ratings, set by the data's size and
-                                n_feat. Speed only.
+                                n_feat. Speed only, but for rounding.
                                 Not used with the per-day terms and for n_feat
                                 of 257 to 2048 (every item takes a block) and
                                 above (every item takes a warp); at most 32768

@@ -31,7 +31,7 @@ constexpr int kCW = 4;                // consumer warps
 constexpr int kPW = 8;                // producer warps
 constexpr int kItemThreads = (kCW + kPW) * 32;
 constexpr int kVecs = 10;             // per-rating vectors of a round
-// FP16 rows of the Gram operands: Fs values + 16 bytes, so that the eight
+// 16-bit rows of the Gram operands: Fs values + 16 bytes, so that the eight
 // 16-byte row segments an ldmatrix reads fall in distinct bank groups
 __host__ __device__ constexpr uint32_t hl_pitch(uint32_t Fs) { return Fs * 2 + 16; }
 static_assert(kPW * 4 == kRound, "each producer warp stages four of the round's ratings");
@@ -46,7 +46,7 @@ __host__ __device__ inline ItemSmem item_smem(uint32_t Fs, uint32_t NF) {
     L.qfs = o;  o += NF * (Fs + 4);             // the item's q^f rows, padded
     L.qsh = o;  o += Fs;                        // q at the round's start
     L.buf = o;  o += 2 * kRound * (Fs + 4);     // two rounds of pe rows + {bu_t, cu_t, res, key}
-    L.hl = o;   o += 2 * kRound * (Fs / 2 + 4); // FP16 high and low parts of the produced round's pe rows
+    L.hl = o;   o += 2 * kRound * (Fs / 2 + 4); // high and low parts of the produced round's pe rows
     L.mbuf = o; o += 2 * kRound * kMS;          // two rounds of the system M (row j: M_j,i)
     L.vec = o;  o += 2 * kVecs * kRound;        // two rounds of per-rating weights
     L.pd = o;   o += kCW * 2 * kRound;          // consumers' partial dots
@@ -169,13 +169,42 @@ __device__ void item_light(const DeviceState& s, const EpochParams& p, const Bf1
     store_item_state(s, i, lane, st);
 }
 
-// One staged rating: its FP32 pe row (for the consumers) and the FP16 high and
-// low parts of it, scaled (the Gram operands), each element split once. Returns the
-// inverse of the scale.
-template <int VPL>
+// Packed BF16 pairs of (x, y): the values rounded, and what that leaves rounded.
+__device__ __forceinline__ void split_pair_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const float2 f = __bfloat1622float2(h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// d (16x8, FP32) += a (16x16, row-major) . b (16x8, column-major), of FP16 or BF16
+template <bool BP>
+__device__ __forceinline__ void mma_parts(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    if constexpr (BP)
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+            "{%0,%1,%2,%3};"
+            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    else mma_f16(d, a, b0, b1);
+}
+
+// One staged rating: its FP32 pe row (for the consumers) and the high and low parts
+// of it (the Gram operands), each element split once: FP16 parts, scaled, and the
+// inverse of the scale is returned, or with `BP` BF16 parts.
+template <int VPL, bool BP>
 __device__ __forceinline__ float stage_row(float* row, uint8_t* hi_row, uint8_t* lo_row, int lane,
                                            const float (&pe)[VPL]) {
-    const float unscale = row_unscale(pe), sc = row_scale(unscale);
+    float unscale = 1.0f, sc = 1.0f;
+    if constexpr (!BP) {
+        unscale = row_unscale(pe);
+        sc = row_scale(unscale);
+    }
+    auto split = [&](float x, float y, uint32_t& h, uint32_t& l) {
+        if constexpr (BP) split_pair_bf16(x, y, h, l);
+        else split_pair(x * sc, y * sc, h, l);
+    };
     if constexpr (VPL % 4 == 0) {
 #pragma unroll
         for (int c = 0; c < VPL / 4; ++c) {
@@ -183,8 +212,8 @@ __device__ __forceinline__ float stage_row(float* row, uint8_t* hi_row, uint8_t*
             const float4 x = make_float4(pe[4 * c], pe[4 * c + 1], pe[4 * c + 2], pe[4 * c + 3]);
             *reinterpret_cast<float4*>(row + col) = x;
             uint2 h, l;
-            split_pair(x.x * sc, x.y * sc, h.x, l.x);
-            split_pair(x.z * sc, x.w * sc, h.y, l.y);
+            split(x.x, x.y, h.x, l.x);
+            split(x.z, x.w, h.y, l.y);
             *reinterpret_cast<uint2*>(hi_row + 2 * col) = h;
             *reinterpret_cast<uint2*>(lo_row + 2 * col) = l;
         }
@@ -193,10 +222,10 @@ __device__ __forceinline__ float stage_row(float* row, uint8_t* hi_row, uint8_t*
         for (int v = 0; v < VPL; ++v) {
             const int col = Row<VPL>::elem(lane, v);
             row[col] = pe[v];
-            const float x = pe[v] * sc;
-            const __half h = __float2half_rn(x);
-            reinterpret_cast<__half*>(hi_row)[col] = h;
-            reinterpret_cast<__half*>(lo_row)[col] = __float2half_rn(x - __half2float(h));
+            uint32_t h, l;
+            split(pe[v], 0.0f, h, l);
+            reinterpret_cast<uint16_t*>(hi_row)[col] = (uint16_t)h;
+            reinterpret_cast<uint16_t*>(lo_row)[col] = (uint16_t)l;
         }
     }
     return unscale;
@@ -210,7 +239,8 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
                  : "r"(addr));
 }
 
-template <int VPL, bool BF>
+// BP: the rounds' dots from BF16 parts (launch_form).
+template <int VPL, bool BF, bool BP>
 __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, EpochParams p, Bf16Copies bf) {
     extern __shared__ __align__(16) float smem[];
     __shared__ uint32_t sh_k;
@@ -356,20 +386,20 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
                     px0[v] = px0[v] + d0 * py0[v];
                     px1[v] = px1[v] + d1 * py1[v];
                 }
-                const float s0 = stage_row<VPL>(dst + (size_t)j0 * stride, hl + (size_t)j0 * hp,
+                const float s0 = stage_row<VPL, BP>(dst + (size_t)j0 * stride, hl + (size_t)j0 * hp,
                                                  hl + (size_t)(kRound + j0) * hp, lane, px0);
-                const float s1 = stage_row<VPL>(dst + (size_t)j1 * stride, hl + (size_t)j1 * hp,
+                const float s1 = stage_row<VPL, BP>(dst + (size_t)j1 * stride, hl + (size_t)j1 * hp,
                                                  hl + (size_t)(kRound + j1) * hp, lane, px1);
 #pragma unroll
                 for (int v = 0; v < VPL; ++v) {
                     x2[v] = x2[v] + d2 * y2[v];
                     x3[v] = x3[v] + d3 * y3[v];
                 }
-                const float s2 = stage_row<VPL>(dst + (size_t)j2 * stride, hl + (size_t)j2 * hp,
+                const float s2 = stage_row<VPL, BP>(dst + (size_t)j2 * stride, hl + (size_t)j2 * hp,
                                                  hl + (size_t)(kRound + j2) * hp, lane, x2);
-                const float s3 = stage_row<VPL>(dst + (size_t)j3 * stride, hl + (size_t)j3 * hp,
+                const float s3 = stage_row<VPL, BP>(dst + (size_t)j3 * stride, hl + (size_t)j3 * hp,
                                                  hl + (size_t)(kRound + j3) * hp, lane, x3);
-                if (lane < 4) V[9 * kRound + pw + kPW * lane] = lane == 0 ? s0 : lane == 1 ? s1 : lane == 2 ? s2 : s3;
+                if (!BP && lane < 4) V[9 * kRound + pw + kPW * lane] = lane == 0 ? s0 : lane == 1 ? s1 : lane == 2 ? s2 : s3;
             }
             // all rows of the round are in place before the Gram products
             asm volatile("bar.sync 2, %0;" ::"r"(kPW * 32) : "memory");
@@ -377,7 +407,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
             // the round's ratings of each frequency bin (valid ratings only)
             const unsigned same = __match_any_sync(kFull, valid ? fbl : 64u + (uint32_t)lane);
             if (pw < 6) {
-                // G = PE PE^T on the tensor cores, from FP16 high and low parts.
+                // G = PE PE^T on the tensor cores, from the rows' high and low parts.
                 // Tile pw of the six 16x8 tiles (rows x columns) that hold
                 // every pair row < column.
                 const int mt = pw < 4 ? 0 : 1, nt = pw < 4 ? pw : pw - 2;
@@ -401,9 +431,9 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
                         ldmatrix_x4(ah, a_hi + kb);
                         ldmatrix_x4(al, a_lo + kb);
                         ldmatrix_x4(bb, b_hl + kb);
-                        mma_f16(d[3 * hh], al, bb[0], bb[1]);
-                        mma_f16(d[3 * hh + 1], ah, bb[2], bb[3]);
-                        mma_f16(d[3 * hh + 2], ah, bb[0], bb[1]);
+                        mma_parts<BP>(d[3 * hh], al, bb[0], bb[1]);
+                        mma_parts<BP>(d[3 * hh + 1], ah, bb[2], bb[3]);
+                        mma_parts<BP>(d[3 * hh + 2], ah, bb[0], bb[1]);
                     }
                 }
                 // The round's errors solve err = C - M err with M unit lower
@@ -419,8 +449,8 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
                     if (ii < jj) {
                         float v = 0.0f;
                         if (jj < (int)m) {
-                            const float g = (((d[0][e] + d[1][e]) + (d[3][e] + d[4][e])) + (d[2][e] + d[5][e])) *
-                                            V[9 * kRound + ii] * V[9 * kRound + jj];
+                            float g = ((d[0][e] + d[1][e]) + (d[3][e] + d[4][e])) + (d[2][e] + d[5][e]);
+                            if constexpr (!BP) g = g * V[9 * kRound + ii] * V[9 * kRound + jj];
                             const float cui = dst[(size_t)ii * stride + Fs + 1], cuj = dst[(size_t)jj * stride + Fs + 1];
                             const bool same_f = rec_fbin(ki) == rec_fbin(kj), same_t = rec_tbin(ki) == rec_tbin(kj);
                             const float bias_lr = p.lr_ib + (same_t ? p.lr_ti : 0.0f) + (same_f ? p.lr_ibf : 0.0f);
@@ -648,9 +678,9 @@ __global__ void __launch_bounds__(kItemThreads, 1) k_item_pass(DeviceState s, Ep
     }
 }
 
-template <int VPL, bool BF>
+template <int VPL, bool BF, bool BP>
 void launch_tiles(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf) {
-    auto kern = k_item_pass<VPL, BF>;
+    auto kern = k_item_pass<VPL, BF, BP>;
     const size_t smem = (size_t)item_smem(s.Fs, s.NF).total * sizeof(float);
     allow_dyn_smem(kern, smem);
     int dev = 0, sms = 0;
@@ -661,20 +691,29 @@ void launch_tiles(tsvd_model* m, const DeviceState& s, const EpochParams& p, con
     m->launches++;
 }
 
-template <int VPL>
+// Items of 32,768 ratings and more have always had their dots from BF16 parts, 16 bits:
+// where no smaller item takes a block they keep them (100,480,507 ratings, f = 256:
+// item pass 59.2 ms, 62.4 from the FP16 parts that the smaller ones need).
+template <int VPL, bool BF>
 void launch_form(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf) {
-    if (bf.pyc) launch_tiles<VPL, true>(m, s, p, bf);
-    else launch_tiles<VPL, false>(m, s, p, bf);
+    if (s.heavy_min >= s.rounded_decay_min) launch_tiles<VPL, BF, true>(m, s, p, bf);
+    else launch_tiles<VPL, BF, false>(m, s, p, bf);
+}
+
+template <int VPL>
+void launch_rows(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf) {
+    if (bf.pyc) launch_form<VPL, true>(m, s, p, bf);
+    else launch_form<VPL, false>(m, s, p, bf);
 }
 
 }  // namespace
 
 void launch_item_tiles(tsvd_model* m, const DeviceState& s, const EpochParams& p, const Bf16Copies& bf) {
     switch (s.Fs / 32) {
-        case 5: launch_form<5>(m, s, p, bf); break;
-        case 6: launch_form<6>(m, s, p, bf); break;
-        case 7: launch_form<7>(m, s, p, bf); break;
-        case 8: launch_form<8>(m, s, p, bf); break;
+        case 5: launch_rows<5>(m, s, p, bf); break;
+        case 6: launch_rows<6>(m, s, p, bf); break;
+        case 7: launch_rows<7>(m, s, p, bf); break;
+        case 8: launch_rows<8>(m, s, p, bf); break;
         default: throw Error(TSVD_ERR_UNSUPPORTED, "item tiles take rows of 160 to 256 columns");
     }
 }

@@ -129,6 +129,7 @@ def test_thresholds_that_take_the_same_items_give_the_same_bits(f):
                 assert np.array_equal(g[n], got[0][n]), (same, n)
 
 
+FROZEN = {n: 0.0 for n in ("lr_u", "lr_u2", "lr_ub", "lr_ubd", "lr_y", "lr_yb", "lr_ta", "lr_tu", "lr_cu")}
 ROUND_COUNTS = [64, 32, 20, 2]
 
 
@@ -203,7 +204,42 @@ def test_a_round_keeps_the_digits_of_its_rows(f, low_memory, ordinal):
             assert np.max(np.abs(got[k, :c] - want)) < (6e-6 if ordinal else 4.8e-6), (heavy, c)
 
 
-FROZEN = {n: 0.0 for n in ("lr_u", "lr_u2", "lr_ub", "lr_ubd", "lr_y", "lr_yb", "lr_ta", "lr_tu", "lr_cu")}
+@pytest.mark.parametrize("f,low_memory", [(20, True), (64, True), (128, True), (160, True), (256, True), (60, False),
+                                          (200, False)])
+def test_rows_far_beyond_the_learning_rate(f, low_memory):
+    """Values of 100 sqrt(2 / lr), far past what FP16 holds without a scale: the second
+    rating's error is that of the 64-bit chain.
+
+    Tolerance: relative, all terms of a score and of a dot have one sign; 20 roundings of
+    2^-24 a score, as many for the first error's way into the second, 64 + 8 for the dot
+    of the rows: 112 x 2^-24 = 7e-6."""
+    u, i = np.array([0, 0, 1, 1, 63]), np.array([0, 1, 0, 1, 2])
+    tr = Dataset.from_ratings(u, i, 1 + (u + i) % 5, 20 * u + i, 64, 4, "large")
+    pr = Dataset.from_ratings(np.arange(64), np.full(64, 3), np.full(64, 3), 20 * np.arange(64) + 9, 64, 4, "large_pr")
+    lr = float(np.float32(0.005))
+    cfg = run_lm(f, 1, n_time_bins=64, low_memory=low_memory).replace(
+        lr_i=lr, lr_iqf=lr, lr_ti=1.0, lr_ib=0.0, lr_ibf=0.0, lr_ud=0.0, lr_yd=0.0, reg_i=0.0, reg_iqf=0.0, **FROZEN)
+    rng = np.random.default_rng(7)
+    nf = cfg.n_freq_bins
+    init = {"ufeat": np.full((64, f), 2000.0, np.float32), "ufeat2": np.zeros((64, f), np.float32),
+            "ifeat": rng.uniform(0.01, 0.02, (4, f)).astype(np.float32), "yfeat": np.zeros((4, f), np.float32),
+            "ifeat_freq": rng.uniform(0.01, 0.02, (4 * nf, f)).astype(np.float32)}
+    if not low_memory:
+        init["yfeat_day"] = np.zeros((4, f), np.float32)
+    for heavy in (1, 100000):
+        m = TxModel(tr, MaskedDataset(pr), cfg, heavy_item_ratings=heavy)
+        for k, v in init.items():
+            m.set_param(k, v)
+        m.fit_epoch(tr, pr, 1)
+        g = float(np.asarray(m.get_param("gbias")).ravel()[0])
+        got = -np.asarray(m.get_param("bit_bin"), np.float64).reshape(4, 64)
+        for k in range(2):
+            y = 1 + (np.arange(2) + k) % 5
+            want = chain_errors(init["ufeat"][:2].astype(np.float64), init["ifeat"][k].astype(np.float64),
+                                init["ifeat_freq"][k * nf].astype(np.float64), y, lr, g, None)
+            assert np.max(np.abs(got[k, :2] / want - 1)) < 7e-6, (heavy, k)
+
+
 # strong updates and decays of rows and bins, as in the tests of the item stratum without the head
 STRONG = dict(lr_ti=0.002, lr_ibf=0.003, lr_iqf=0.004, reg_iqf=0.05, reg_i=0.05, sigma_u=0.1, sigma_i=0.1, sigma_iqf=0.1)
 
